@@ -219,7 +219,7 @@ __global__ void batch_init_rows_kernel(BatchArgs a, int slot0) {
 }
 
 // Loads plant `pi` into the block's shared DevPlant and stages its statics.
-template <bool SM>
+template <int M>
 static __device__ bool block_plant(const BatchArgs& a, int pi, DevPlant* sp, int* cur, float4* smem4, uint64_t* bar) {
   if (*cur == pi) return true;
   __syncthreads();
@@ -228,31 +228,25 @@ static __device__ bool block_plant(const BatchArgs& a, int pi, DevPlant* sp, int
     *cur = pi;
   }
   __syncthreads();
-  if (SM) return stage_statics(*sp, smem4, bar);
+  if (M == kModeStaged) return stage_statics(*sp, smem4, bar);
   return true;
 }
 
-template <bool SM>
-static __device__ __forceinline__ WarpCtx<SM> batch_ctx(const DevPlant& p, float4* smem4, int static_floats) {
-  WarpCtx<SM> w;
-  const int warp = threadIdx.x >> 5;
+template <int M>
+static __device__ __forceinline__ WarpCtx<M> batch_ctx(const DevPlant& p, float4* smem4, int static_floats) {
+  WarpCtx<M> w;
   w.ok = true;
-  w.stat = SM ? smem4 : p.statics;
-  w.aabb = SM ? smem4 + 4 * p.num_static : p.aabb;
-  float* wbase = reinterpret_cast<float*>(smem4) + (SM ? static_floats : 0);
-  w.X = wbase + warp * warp_floats(p);
-  w.qs = w.X + p.num_slots * 12;
-  w.q1 = w.qs + kMaxDim;
-  w.q2 = w.q1 + kMaxDim;
-  w.pose = w.q2 + kMaxDim;
+  w.stat = M == kModeStaged ? smem4 : p.statics;
+  w.aabb = M == kModeStaged ? smem4 + 4 * p.num_static : p.aabb;
+  warp_buffers<M>(p, reinterpret_cast<float*>(smem4) + static_floats, w);
   return w;
 }
 
 // Work item = (active slot, chunk of configurations), sized so that the grid
 // gets about four items per block whether 256 slots or one are active; items
 // are handed out by the work queue it->check_next (plants differ in cost).
-template <bool SM>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) batch_check_kernel(BatchArgs a, int static_floats) {
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) batch_check_kernel(BatchArgs a, int static_floats) {
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
   __shared__ DevPlant sp;
@@ -271,16 +265,15 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) batch_check_kernel(Bat
     const SlotState& S = a.slots[slot];
     const int Ns = a.n_tab[S.k];
     if (first >= Ns) continue;  // uniform across the block
-    if (!block_plant<SM>(a, S.plant, &sp, &cur, smem4, &bar)) return;
-    const WarpCtx<SM> w = batch_ctx<SM>(sp, smem4, static_floats);
+    if (!block_plant<M>(a, S.plant, &sp, &cur, smem4, &bar)) return;
+    const WarpCtx<M> w = batch_ctx<M>(sp, smem4, static_floats);
     const float* smp = a.fpool + S.smp_off;
     uint8_t* flags = a.bpool + S.flag_off;
     const int last = std::min(Ns, first + c);
     for (int i = first + warp; i < last; i += nw) {
       if (lane < sp.dim) w.qs[lane] = smp[(int64_t)i * sp.dim + lane];
       __syncwarp();
-      fk_warp(sp, w.qs, w.X, lane);
-      const bool hit = check_config(sp, w.stat, w.aabb, w.X, w.pose, lane, none);
+      const bool hit = check_warp<M>(sp, w, lane, none);
       if (lane == 0) flags[i] = hit ? 0 : 1;
     }
   }
@@ -311,8 +304,8 @@ __global__ void __launch_bounds__(1024) batch_compact_kernel(BatchArgs a) {
   }
 }
 
-template <bool SM>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) batch_bisect_kernel(BatchArgs a, int static_floats) {
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) batch_bisect_kernel(BatchArgs a, int static_floats) {
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
   __shared__ DevPlant sp;
@@ -330,12 +323,12 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) batch_bisect_kernel(Ba
     const int slot = a.act[it / ips], first = (it % ips) * c;
     const SlotState& S = a.slots[slot];
     if (S.done || first >= S.K) continue;  // uniform across the block
-    if (!block_plant<SM>(a, S.plant, &sp, &cur, smem4, &bar)) return;
-    const WarpCtx<SM> w = batch_ctx<SM>(sp, smem4, static_floats);
+    if (!block_plant<M>(a, S.plant, &sp, &cur, smem4, &bar)) return;
+    const WarpCtx<M> w = batch_ctx<M>(sp, smem4, static_floats);
     const float* ls = a.fpool + S.seg_off;
     const int last = std::min(S.K, first + c);
     for (int i = first + warp; i < last; i += nw)
-      bisect_particle<SM>(sp, w, i, S.dim, a.bisection, ls, ls + S.dim, none, a.fpool + S.col_off,
+      bisect_particle<M>(sp, w, i, S.dim, a.bisection, ls, ls + S.dim, none, a.fpool + S.col_off,
                           a.fpool + S.col_off + (int64_t)a.num_particles * S.dim, a.fpool + S.dist_off, lane);
   }
 }
@@ -514,8 +507,8 @@ __global__ void __launch_bounds__(1024) batch_sort_kernel(BatchArgs a) {
 // Round r of the sorted check: the positions of round r of every slot that
 // still needs checking, in (slot, chunk) items from the work queue as
 // batch_check_kernel.
-template <bool SM>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) batch_check_sorted_kernel(BatchArgs a, int static_floats,
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) batch_check_sorted_kernel(BatchArgs a, int static_floats,
                                                                                    int r) {
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
@@ -538,8 +531,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) batch_check_sorted_ker
     const SlotState& S = a.slots[slot];
     const int Ns = a.n_tab[S.k], end_s = round_end(a, r, Ns), first = round_begin(a, r, Ns) + (it % ips) * c;
     if (S.done || !S.need || first >= end_s) continue;  // uniform across the block
-    if (!block_plant<SM>(a, S.plant, &sp, &cur, smem4, &bar)) return;
-    const WarpCtx<SM> w = batch_ctx<SM>(sp, smem4, static_floats);
+    if (!block_plant<M>(a, S.plant, &sp, &cur, smem4, &bar)) return;
+    const WarpCtx<M> w = batch_ctx<M>(sp, smem4, static_floats);
     const float* smp = a.fpool + S.smp_off;
     const int* ord = a.order + (size_t)slot * a.n_max;
     uint8_t* flags = a.bpool + S.flag_off;
@@ -548,8 +541,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) batch_check_sorted_ker
       const int i = ord[p];
       if (lane < sp.dim) w.qs[lane] = smp[(int64_t)i * sp.dim + lane];
       __syncwarp();
-      fk_warp(sp, w.qs, w.X, lane);
-      const bool hit = check_config(sp, w.stat, w.aabb, w.X, w.pose, lane, none);
+      const bool hit = check_warp<M>(sp, w, lane, none);
       if (lane == 0) flags[i] = hit ? 0 : 1;
     }
   }
@@ -707,7 +699,7 @@ struct csd_batch_s {
   std::vector<csd_plant_t> plants;
   csd_eizo_options_t opt{};
   int max_slots = 0, capacity = 0, n_max = 0, max_dim = 0;
-  bool sm = true;
+  int mode = csd::kModeStaged;   // how configurations are checked (check_warp.cuh), one for all plants
   int static_floats = 0;
   size_t check_smem = 0;
   int check_grid = 0, bisect_grid = 0;
@@ -795,6 +787,14 @@ int variant_for(const csd_batch_s* h, int nf8, int nf16) {
   return best;
 }
 
+void launch_check(const csd_batch_s* h, const BatchArgs& a, cudaStream_t s) {
+  with_mode(h->mode, [&](auto m) -> csd_status_t {
+    batch_check_kernel<decltype(m)::value>
+        <<<h->check_grid, 32 * kWarpsPerBlock, h->check_smem, s>>>(a, h->static_floats);
+    return CSD_OK;
+  });
+}
+
 // One iteration's launches on stream s. ev (kStages + 1 events) brackets the
 // stages for the profiling mode; skip_sample leaves out the sampler (the
 // autotuner has just run it).
@@ -814,11 +814,11 @@ int launch_iteration(csd_batch_s* h, int num_slots, const BatchArgs& a, cudaStre
     if (ev) cudaEventRecord(ev[3], s);
     for (int r = 0; r < a.rounds; ++r) {
       cudaMemsetAsync(&a.it->check_next, 0, sizeof(int), s);
-      if (h->sm)
-        batch_check_sorted_kernel<true><<<h->check_grid, 32 * kWarpsPerBlock, h->check_smem, s>>>(a, h->static_floats,
-                                                                                                  r);
-      else
-        batch_check_sorted_kernel<false><<<h->check_grid, 32 * kWarpsPerBlock, h->check_smem, s>>>(a, 0, r);
+      with_mode(h->mode, [&](auto m) -> csd_status_t {
+        batch_check_sorted_kernel<decltype(m)::value>
+            <<<h->check_grid, 32 * kWarpsPerBlock, h->check_smem, s>>>(a, h->static_floats, r);
+        return CSD_OK;
+      });
       batch_tally_kernel<<<num_slots, 256, 0, s>>>(a, r);
     }
     if (ev) cudaEventRecord(ev[4], s);
@@ -827,19 +827,17 @@ int launch_iteration(csd_batch_s* h, int num_slots, const BatchArgs& a, cudaStre
     if (ev) cudaEventRecord(ev[2], s);
     if (ev) cudaEventRecord(ev[3], s);
     cudaMemsetAsync(&a.it->check_next, 0, sizeof(int), s);
-    if (h->sm)
-      batch_check_kernel<true><<<h->check_grid, 32 * kWarpsPerBlock, h->check_smem, s>>>(a, h->static_floats);
-    else
-      batch_check_kernel<false><<<h->check_grid, 32 * kWarpsPerBlock, h->check_smem, s>>>(a, 0);
+    launch_check(h, a, s);
     if (ev) cudaEventRecord(ev[4], s);
     batch_compact_kernel<<<num_slots, 1024, 0, s>>>(a);
   }
   if (ev) cudaEventRecord(ev[5], s);
   cudaMemsetAsync(&a.it->bisect_next, 0, sizeof(int), s);
-  if (h->sm)
-    batch_bisect_kernel<true><<<h->bisect_grid, 32 * kWarpsPerBlock, h->check_smem, s>>>(a, h->static_floats);
-  else
-    batch_bisect_kernel<false><<<h->bisect_grid, 32 * kWarpsPerBlock, h->check_smem, s>>>(a, 0);
+  with_mode(h->mode, [&](auto m) -> csd_status_t {
+    batch_bisect_kernel<decltype(m)::value>
+        <<<h->bisect_grid, 32 * kWarpsPerBlock, h->check_smem, s>>>(a, h->static_floats);
+    return CSD_OK;
+  });
   if (ev) cudaEventRecord(ev[6], s);
   batch_faces_kernel<<<num_slots, 1024, 0, s>>>(a);
   if (ev) cudaEventRecord(ev[7], s);
@@ -908,7 +906,8 @@ csd_status_t csd_batch_create(const csd_plant_t* plants, int32_t num_plants, int
   h->opt = *o;
   h->max_slots = max_slots;
   h->capacity = face_capacity;
-  int max_static = 0, max_wf = 0;
+  int max_static = 0, max_wf = 0, max_field_wf = 0;
+  bool field = true;  // every plant has the field tables and its broad phase on
   std::vector<DevPlant> dps;
   for (int i = 0; i < num_plants; ++i) {
     CSD_CHECK(plants[i] && plants[i]->device == h->device, CSD_ERR_INVALID, "plants must live on one device");
@@ -918,6 +917,8 @@ csd_status_t csd_batch_create(const csd_plant_t* plants, int32_t num_plants, int
     h->max_dim = std::max(h->max_dim, plants[i]->dp.dim);
     max_static = std::max(max_static, plants[i]->dp.static_bytes);
     max_wf = std::max(max_wf, warp_floats(plants[i]->dp));
+    max_field_wf = std::max(max_field_wf, field_warp_floats(plants[i]->dp));
+    field = field && plant_mode(plants[i]) == kModeField;
   }
   // iteration tables (cuda_edge_inflation_zero_order.cu:113-119)
   for (uint32_t k = 0; k < o->max_iterations; ++k) {
@@ -931,21 +932,18 @@ csd_status_t csd_batch_create(const csd_plant_t* plants, int32_t num_plants, int
   // the stage kernels number their work items (slot, 8 or more configurations) with 32-bit integers
   CSD_CHECK((int64_t)max_slots * (h->n_max / 8 + 1) + (1 << 20) < (int64_t)INT32_MAX, CSD_ERR_CAPACITY,
             "too many slots times samples per iteration");
-  h->sm = max_static <= kStaticSmemLimit;
-  h->static_floats = h->sm ? max_static / 4 : 0;
-  h->check_smem = (size_t)max_wf * sizeof(float) * kWarpsPerBlock + (h->sm ? (size_t)max_static : 0);
-  csd_status_t s;
-  int g1 = 0, g2 = 0;
-  int g3 = 0;
-  if (h->sm) {
-    if ((s = grid_for(batch_check_kernel<true>, h->check_smem, 1ll << 40, &g1, kWarpsPerBlock))) return s;
-    if ((s = grid_for(batch_bisect_kernel<true>, h->check_smem, 1ll << 40, &g2, kWarpsPerBlock))) return s;
-    if ((s = grid_for(batch_check_sorted_kernel<true>, h->check_smem, 1ll << 40, &g3, kWarpsPerBlock))) return s;
-  } else {
-    if ((s = grid_for(batch_check_kernel<false>, h->check_smem, 1ll << 40, &g1, kWarpsPerBlock))) return s;
-    if ((s = grid_for(batch_bisect_kernel<false>, h->check_smem, 1ll << 40, &g2, kWarpsPerBlock))) return s;
-    if ((s = grid_for(batch_check_sorted_kernel<false>, h->check_smem, 1ll << 40, &g3, kWarpsPerBlock))) return s;
-  }
+  h->mode = field ? kModeField : max_static <= kStaticSmemLimit ? kModeStaged : kModeGlobal;
+  h->static_floats = h->mode == kModeStaged ? max_static / 4 : 0;
+  h->check_smem = (size_t)(field ? max_field_wf : max_wf) * sizeof(float) * kWarpsPerBlock +
+                  (size_t)h->static_floats * sizeof(float);
+  int g1 = 0, g2 = 0, g3 = 0;
+  csd_status_t s = with_mode(h->mode, [&](auto m) -> csd_status_t {
+    constexpr int kM = decltype(m)::value;
+    if (csd_status_t e = grid_for(batch_check_kernel<kM>, h->check_smem, 1ll << 40, &g1, kWarpsPerBlock)) return e;
+    if (csd_status_t e = grid_for(batch_bisect_kernel<kM>, h->check_smem, 1ll << 40, &g2, kWarpsPerBlock)) return e;
+    return grid_for(batch_check_sorted_kernel<kM>, h->check_smem, 1ll << 40, &g3, kWarpsPerBlock);
+  });
+  if (s) return s;
   h->check_grid = g1;
   h->bisect_grid = g2;
   for (int v = 0; v < kNumSampleVariants; ++v) {
@@ -1215,10 +1213,7 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
         ac.cfg_max = kCheckItemCaps[c];
         cudaMemsetAsync(&a.it->check_next, 0, sizeof(int), st);
         cudaEventRecord(tev[2 * j], st);
-        if (h->sm)
-          batch_check_kernel<true><<<h->check_grid, 32 * kWarpsPerBlock, h->check_smem, st>>>(ac, h->static_floats);
-        else
-          batch_check_kernel<false><<<h->check_grid, 32 * kWarpsPerBlock, h->check_smem, st>>>(ac, 0);
+        launch_check(h, ac, st);
         cudaEventRecord(tev[2 * j + 1], st);
         ++h->launches;
       }

@@ -13,25 +13,24 @@
 // and the verdict bytes touch HBM.
 #include <algorithm>
 
-#include "check_core.cuh"
+#include "check_warp.cuh"
 
 namespace csd {
 
-template <bool SM>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) check_points_kernel(DevPlant p, const float* __restrict__ q,
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) check_points_kernel(DevPlant p, const float* __restrict__ q,
                                                                           int64_t n, VoxArgs va,
                                                                           uint8_t* __restrict__ out) {
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
-  const WarpCtx<SM> w = warp_setup<SM>(p, smem4, &bar);
+  const WarpCtx<M> w = warp_setup<M>(p, smem4, &bar);
   if (!w.ok) return;
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += nw) {
     if (lane < p.dim) w.qs[lane] = q[i * p.dim + lane];
     __syncwarp();
-    fk_warp(p, w.qs, w.X, lane);
-    const bool hit = check_config(p, w.stat, w.aabb, w.X, w.pose, lane, va);
+    const bool hit = check_warp<M>(p, w, lane, va);
     if (lane == 0) out[i] = hit ? 0 : 1;
   }
 }
@@ -121,8 +120,8 @@ static __device__ __forceinline__ void edge_pair(int64_t e, int64_t n, int64_t* 
 
 // nodes > 0: the edges are every pair i < j of the `nodes` configurations in
 // `starts` (ends unused), in upper-triangle row-major order.
-template <bool SM>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) check_edges_kernel(DevPlant p, const float* __restrict__ starts,
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) check_edges_kernel(DevPlant p, const float* __restrict__ starts,
                                                                          const float* __restrict__ ends, int64_t n,
                                                                          float step, int mode,
                                                                          uint8_t* __restrict__ out,
@@ -130,7 +129,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) check_edges_kernel(Dev
                                                                          unsigned long long* counter, int64_t nodes) {
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
-  const WarpCtx<SM> w = warp_setup<SM>(p, smem4, &bar);
+  const WarpCtx<M> w = warp_setup<M>(p, smem4, &bar);
   if (!w.ok) return;
   const int lane = threadIdx.x & 31;
   const int d = p.dim;
@@ -165,9 +164,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) check_edges_kernel(Dev
       __syncwarp();
       if (lane < d) w.qs[lane] = x;
       __syncwarp();
-      fk_warp(p, w.qs, w.X, lane);
       ++checked;
-      collided = check_config(p, w.stat, w.aabb, w.X, w.pose, lane, none);
+      collided = check_warp<M>(p, w, lane, none);
     }
     if (lane == 0) {
       out[e] = collided ? 0 : 1;
@@ -205,15 +203,15 @@ __global__ void edge_materialize_kernel(const float* __restrict__ s, const float
 // coarse-to-fine as check_edges_kernel visits them. The verdict is the AND
 // over all points either way; only the order (and so the early exit) depends
 // on the logits.
-template <bool SM>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3)
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n)
     check_edges_ranked_kernel(DevPlant p, const float* __restrict__ starts, const float* __restrict__ ends, int64_t e0,
                               int64_t e1, const int64_t* __restrict__ off, const float* __restrict__ logits, int top,
                               int mode, uint8_t* __restrict__ out, int64_t* __restrict__ pts,
                               unsigned long long* counter) {
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
-  const WarpCtx<SM> w = warp_setup<SM>(p, smem4, &bar);
+  const WarpCtx<M> w = warp_setup<M>(p, smem4, &bar);
   if (!w.ok) return;
   const int lane = threadIdx.x & 31;
   const int d = p.dim;
@@ -286,9 +284,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 3)
       __syncwarp();
       if (lane < d) w.qs[lane] = x;
       __syncwarp();
-      fk_warp(p, w.qs, w.X, lane);
       ++checked;
-      collided = check_config(p, w.stat, w.aabb, w.X, w.pose, lane, none);
+      collided = check_warp<M>(p, w, lane, none);
     }
     if (lane == 0) {
       out[e] = collided ? 0 : 1;
@@ -303,7 +300,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) fk_kernel(DevPlant p, con
                                                                 float* __restrict__ tf_out) {
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
-  const WarpCtx<false> w = warp_setup<false>(p, smem4, &bar);
+  const WarpCtx<kModeGlobal> w = warp_setup<kModeGlobal>(p, smem4, &bar);
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += nw) {
@@ -345,36 +342,26 @@ __global__ void pair_kernel(int ta, const float* g, int tb, uint8_t* out) {
 }
 
 // ----------------------------------------------------------------- launchers
-template <typename K>
-static csd_status_t launch_grid(const csd_plant_s* p, K kernel, bool sm, int64_t work_warps, size_t* smem, int* grid) {
-  *smem = (size_t)warp_floats(p->dp) * sizeof(float) * kWarpsPerBlock + (sm ? (size_t)p->dp.static_bytes : 0);
-  return grid_for(kernel, *smem, work_warps, grid, kWarpsPerBlock);
-}
-
 csd_status_t launch_check_points(const csd_plant_s* p, const float* q, int64_t n, const VoxelTables& vt,
                                  uint8_t* out, cudaStream_t st) {
   if (n <= 0) return CSD_OK;
   const VoxArgs va = vox_args(vt);
-  size_t smem = 0;
-  int grid = 0;
-  csd_status_t s;
-  if (statics_in_smem(p)) {
-    if ((s = launch_grid(p, check_points_kernel<true>, true, n, &smem, &grid))) return s;
-    check_points_kernel<true><<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, q, n, va, out);
-  } else {
-    if ((s = launch_grid(p, check_points_kernel<false>, false, n, &smem, &grid))) return s;
-    check_points_kernel<false><<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, q, n, va, out);
-  }
-  CSD_CUDA_TRY(cudaGetLastError());
-  return CSD_OK;
+  return with_mode(plant_mode(p), [&](auto m) -> csd_status_t {
+    auto kernel = check_points_kernel<decltype(m)::value>;
+    const size_t smem = smem_bytes(p, kWarpsPerBlock);
+    int grid = 0;
+    if (csd_status_t s = grid_for(kernel, smem, n, &grid, kWarpsPerBlock)) return s;
+    kernel<<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, q, n, va, out);
+    CSD_CUDA_TRY(cudaGetLastError());
+    return CSD_OK;
+  });
 }
 
 csd_status_t launch_fk(const csd_plant_s* p, const float* q, int64_t n, float* tf, cudaStream_t st) {
   if (n <= 0) return CSD_OK;
-  size_t smem = 0;
+  const size_t smem = (size_t)warp_floats(p->dp) * sizeof(float) * kWarpsPerBlock;
   int grid = 0;
-  csd_status_t s = launch_grid(p, fk_kernel, false, n, &smem, &grid);
-  if (s) return s;
+  if (csd_status_t s = grid_for(fk_kernel, smem, n, &grid, kWarpsPerBlock)) return s;
   fk_kernel<<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, q, n, tf);
   CSD_CUDA_TRY(cudaGetLastError());
   return CSD_OK;
@@ -402,44 +389,34 @@ csd_status_t launch_check_edges_ranked(const csd_plant_s* p, const float* s0, co
                                        const int64_t* off, const float* logits, int top, int mode, uint8_t* out,
                                        int64_t* pts, unsigned int* counter, cudaStream_t st) {
   if (e1 <= e0) return CSD_OK;
-  size_t smem = 0;
-  int grid = 0;
-  csd_status_t s;
   CSD_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
   unsigned long long* ctr = reinterpret_cast<unsigned long long*>(counter);
-  if (statics_in_smem(p)) {
-    if ((s = launch_grid(p, check_edges_ranked_kernel<true>, true, e1 - e0, &smem, &grid))) return s;
-    check_edges_ranked_kernel<true><<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, s0, e0p, e0, e1, off, logits, top,
-                                                                              mode, out, pts, ctr);
-  } else {
-    if ((s = launch_grid(p, check_edges_ranked_kernel<false>, false, e1 - e0, &smem, &grid))) return s;
-    check_edges_ranked_kernel<false><<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, s0, e0p, e0, e1, off, logits,
-                                                                               top, mode, out, pts, ctr);
-  }
-  CSD_CUDA_TRY(cudaGetLastError());
-  return CSD_OK;
+  return with_mode(plant_mode(p), [&](auto m) -> csd_status_t {
+    auto kernel = check_edges_ranked_kernel<decltype(m)::value>;
+    const size_t smem = smem_bytes(p, kWarpsPerBlock);
+    int grid = 0;
+    if (csd_status_t s = grid_for(kernel, smem, e1 - e0, &grid, kWarpsPerBlock)) return s;
+    kernel<<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, s0, e0p, e0, e1, off, logits, top, mode, out, pts, ctr);
+    CSD_CUDA_TRY(cudaGetLastError());
+    return CSD_OK;
+  });
 }
 
 csd_status_t launch_check_edges(const csd_plant_s* p, const float* s0, const float* e0, int64_t n, float step,
                                 int mode, uint8_t* out, int64_t* pts, unsigned int* counter, cudaStream_t st,
                                 int64_t nodes) {
   if (n <= 0) return CSD_OK;
-  size_t smem = 0;
-  int grid = 0;
-  csd_status_t s;
   CSD_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
   unsigned long long* ctr = reinterpret_cast<unsigned long long*>(counter);
-  if (statics_in_smem(p)) {
-    if ((s = launch_grid(p, check_edges_kernel<true>, true, n, &smem, &grid))) return s;
-    check_edges_kernel<true><<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, s0, e0, n, step, mode, out, pts, ctr,
-                                                                       nodes);
-  } else {
-    if ((s = launch_grid(p, check_edges_kernel<false>, false, n, &smem, &grid))) return s;
-    check_edges_kernel<false><<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, s0, e0, n, step, mode, out, pts, ctr,
-                                                                        nodes);
-  }
-  CSD_CUDA_TRY(cudaGetLastError());
-  return CSD_OK;
+  return with_mode(plant_mode(p), [&](auto m) -> csd_status_t {
+    auto kernel = check_edges_kernel<decltype(m)::value>;
+    const size_t smem = smem_bytes(p, kWarpsPerBlock);
+    int grid = 0;
+    if (csd_status_t s = grid_for(kernel, smem, n, &grid, kWarpsPerBlock)) return s;
+    kernel<<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, s0, e0, n, step, mode, out, pts, ctr, nodes);
+    CSD_CUDA_TRY(cudaGetLastError());
+    return CSD_OK;
+  });
 }
 
 csd_status_t launch_pair(int ta, const float* g_dev, int tb, uint8_t* out, cudaStream_t st) {

@@ -872,65 +872,4 @@ static __device__ bool check_config(const DevPlant& p, const float4* stat, const
   return false;
 }
 
-// Shared-memory setup common to the warp-per-configuration kernels. SM: the
-// static tables are staged into shared memory.
-template <bool SM>
-struct WarpCtx {
-  const float4* stat;
-  const float4* aabb;
-  float* X;
-  float* qs;
-  float* q1;
-  float* q2;
-  float* pose;
-  bool ok;
-};
-
-template <bool SM>
-static __device__ __forceinline__ WarpCtx<SM> warp_setup(const DevPlant& p, float4* smem4, uint64_t* bar) {
-  WarpCtx<SM> w;
-  const int warp = threadIdx.x >> 5;
-  float* wbase;
-  if (SM) {
-    w.ok = stage_statics(p, smem4, bar);
-    w.stat = smem4;
-    w.aabb = smem4 + 4 * p.num_static;
-    wbase = reinterpret_cast<float*>(smem4) + p.static_bytes / 4;
-  } else {
-    w.ok = true;
-    w.stat = p.statics;
-    w.aabb = p.aabb;
-    wbase = reinterpret_cast<float*>(smem4);
-  }
-  w.X = wbase + warp * warp_floats(p);
-  w.qs = w.X + p.num_slots * 12;
-  w.q1 = w.qs + kMaxDim;
-  w.q2 = w.q1 + kMaxDim;
-  w.pose = w.q2 + kMaxDim;
-  return w;
-}
-
-// ---- host helpers shared by the launchers
-static inline bool statics_in_smem(const csd_plant_s* p) { return p->dp.static_bytes <= kStaticSmemLimit; }
-
-static inline size_t smem_bytes(const csd_plant_s* p, int wpb) {
-  size_t per = (size_t)warp_floats(p->dp) * sizeof(float) * wpb;
-  return per + (statics_in_smem(p) ? (size_t)p->dp.static_bytes : 0);
-}
-
-template <typename K>
-static csd_status_t grid_for(K kernel, size_t smem, int64_t work_warps, int* grid, int wpb) {
-  int per_sm = 0;
-  CSD_CUDA_TRY(raise_smem_limit(kernel, (int)smem));
-  CSD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * wpb, smem));
-  if (per_sm <= 0) {
-    set_error("plant tables do not fit in shared memory");
-    return CSD_ERR_CAPACITY;
-  }
-  int64_t need = (work_warps + wpb - 1) / wpb;
-  int64_t full = (int64_t)per_sm * device_sm_count();
-  *grid = (int)std::max<int64_t>(1, std::min(need, full));
-  return CSD_OK;
-}
-
 }  // namespace csd

@@ -87,6 +87,43 @@ struct TileEntry {    // one static geometry (or moving partner) and the lanes o
   uint32_t mask;
 };
 
+// ---- tables of the field path (check_field.cuh): plants whose moving
+// geometries are spheres and capsules.
+struct LinkPair {     // moving-moving pairs of slots sa and sb: sphere-sphere, sphere-capsule, capsule-capsule
+  int sa, sb;
+  int begin;          // first entry of FieldTables::pairs
+  int nss, nsc, ncc;
+};
+
+struct FieldTables {
+  // Cells over the world statics. A cell lists the statics within
+  // max_r + half a cell diagonal (padded) of its centre: no other static can
+  // touch a probe of radius <= max_r whose centre lies in the cell.
+  const uint4* cells;       // x: distance of the centre to the nearest listed static (binary16, rounded down,
+                            // capped) | number of statics << 16 (0xffff: test every static); y, z, w: up to
+                            // six 16-bit static indices, or (more than six) y = first entry of `list`
+  const uint16_t* list;     // indices of the cells with more than six statics
+  float ox, oy, oz;         // corner of the grid
+  float inv_h, h;           // 1 / cell edge, cell edge
+  int nx, ny, nz;           // 0: no statics
+  float far_lo[3], far_hi[3];  // a probe centre outside this box touches no static
+  const float4* rounded;    // [num_static][2]: sphere or aligned box as [centre radius | half extents 0];
+                            // w of the second float4: 1 rotated box, 2 capsule (WG pose in DevPlant::statics)
+  const uint32_t* pair_bits;  // [num_moving][pair_words] statics each moving geometry pairs with; null: all
+  int pair_words;
+  const float4* geom;       // [num_moving]: centre in the slot frame, radius
+  const float4* cap_axis;   // [num_mcap]: axis in the slot frame, half length
+  const float4* probes;     // [num_probes] of the moving capsules: offset along the axis, radius, capsule (int bits)
+  int num_probes;
+  const float4* link_cap;   // [num_slots][2]: capsule around the slot's geometry (slot frame), radius < 0: none
+  const LinkPair* link_pairs;
+  int num_link_pairs;
+  const uint32_t* pairs;    // moving-moving pairs a | b << 16 by link pair
+  const float4* fk_entry;   // [num_fk][12]: joint-local transform entries (A, B, C, kind), see fk_rows
+  const uint32_t* fk_step;  // [num_steps][8]: joint of each lane group and its parent, see fk_rows
+  int num_steps;
+};
+
 // Plant description passed to kernels by value (pointers are device memory).
 struct DevPlant {
   int dim;
@@ -125,6 +162,8 @@ struct DevPlant {
   const int* link_slot;        // [num_links] slot of each reference link (-1 world, -2 unreachable)
   const float* link_fixed;     // [num_links][12] slot->link (R col-major 9, t 3); world links: world pose
   int* status;                 // device error word: nonzero after a bounded wait gave up
+  int has_field;               // the field tables exist (used while `cull` is on)
+  FieldTables field;
 };
 
 // ------------------------------------------------------------------ FK

@@ -84,6 +84,7 @@ struct csd_plant_s {
   csd::DevPlant dp{};
   csd::HostPlant host;
   void* blob = nullptr;  // device tables
+  void* field_blob = nullptr;  // device tables of the field path (field.cu)
   bool cull_eligible = false;  // <= 32 slots and <= 1024 statics
   bool vox_grid = true;        // voxel checks through the hash grid (csd_plant_set_voxel_grid)
   // scratch for host-pointer calls and per-call voxel tables
@@ -110,6 +111,14 @@ struct VoxelTables {
 
 csd_status_t build_voxel_tables(csd_plant_s* p, const int32_t* robot_ids, int nr, std::vector<uint32_t>* tab,
                                 int* num_other);
+// Tables of the field path (field.cu, check_field.cuh), built by csd_plant_create
+// from the uploaded plant: moving-moving pairs (a | b << 16), the bits of the
+// moving x static pairs, the statics as rounded boxes, the statics' box and
+// the box the robot's geometry stays in (lo[3], hi[3] each). Leaves
+// dp.has_field 0 where the plant does not qualify.
+csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const std::vector<uint32_t>& moving_pairs,
+                         const std::vector<uint32_t>& world_bits, const std::vector<float>& rounded,
+                         const std::vector<double>& static_box, const std::vector<double>& reach_box);
 // Synchronises st, then reads and clears the plant's status word (capi.cu):
 // CSD_ERR_CUDA when a block's bounded staging wait gave up since the last read.
 csd_status_t plant_status(const csd_plant_s* p, cudaStream_t st);

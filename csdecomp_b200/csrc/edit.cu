@@ -37,20 +37,20 @@ namespace csd {
 constexpr int kEditFaceThreads = 256;
 constexpr int kEditMaxVoxels = 10000;  // MAX_NUM_VOXELS, cuda_edge_inflation_zero_order.h:13
 
-template <bool SM>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3)
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n)
     edit_bisect_kernel(DevPlant p, int K, int dim, int steps, const float* __restrict__ starts,
                        const float* __restrict__ ends, const uint32_t* __restrict__ seg, VoxArgs va,
                        float* __restrict__ cols, float* __restrict__ proj, float* __restrict__ dist) {
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
-  const WarpCtx<SM> w = warp_setup<SM>(p, smem4, &bar);
+  const WarpCtx<M> w = warp_setup<M>(p, smem4, &bar);
   if (!w.ok) return;
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
   for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < K; i += nw) {
     const size_t s = (size_t)seg[i] * dim;
-    bisect_particle<SM>(p, w, i, dim, steps, starts + s, ends + s, va, cols, proj, dist, lane);
+    bisect_particle<M>(p, w, i, dim, steps, starts + s, ends + s, va, cols, proj, dist, lane);
   }
 }
 
@@ -314,18 +314,15 @@ csd_status_t csd_edit_regions(csd_plant_t plant, const float* collisions, const 
 
   // 1. bisection, one warp per collision
   const int K = (int)n, steps = (int)options->bisection_steps;
-  const bool sm = statics_in_smem(plant);
-  const size_t smem = smem_bytes(plant, kWarpsPerBlock);
-  int grid = 0;
-  if (sm) {
-    if ((s = grid_for(edit_bisect_kernel<true>, smem, K, &grid, kWarpsPerBlock))) return s;
-    edit_bisect_kernel<true><<<grid, 32 * kWarpsPerBlock, smem, st>>>(plant->dp, K, d, steps, ls, le, seg, va, cols,
-                                                                      proj, dist);
-  } else {
-    if ((s = grid_for(edit_bisect_kernel<false>, smem, K, &grid, kWarpsPerBlock))) return s;
-    edit_bisect_kernel<false><<<grid, 32 * kWarpsPerBlock, smem, st>>>(plant->dp, K, d, steps, ls, le, seg, va,
-                                                                       cols, proj, dist);
-  }
+  s = with_mode(plant_mode(plant), [&](auto md) -> csd_status_t {
+    auto kernel = edit_bisect_kernel<decltype(md)::value>;
+    const size_t smem = smem_bytes(plant, kWarpsPerBlock);
+    int grid = 0;
+    if (csd_status_t e = grid_for(kernel, smem, K, &grid, kWarpsPerBlock)) return e;
+    kernel<<<grid, 32 * kWarpsPerBlock, smem, st>>>(plant->dp, K, d, steps, ls, le, seg, va, cols, proj, dist);
+    return CSD_OK;
+  });
+  if (s) return s;
   CSD_CUDA_TRY(cudaGetLastError());
   // 2. faces, one warp per region
   const int fgrid = std::min((m + kEditFaceThreads / 32 - 1) / (kEditFaceThreads / 32), 8 * device_sm_count());

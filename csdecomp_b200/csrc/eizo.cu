@@ -43,8 +43,8 @@ __global__ void compact_kernel(const uint8_t* __restrict__ flags, const float* _
   compact_block(flags, samples, N, M, max_keep, dim, cols, cnt);
 }
 
-template <bool SM>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) bisect_kernel(DevPlant p, int K, int dim, int steps,
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) bisect_kernel(DevPlant p, int K, int dim, int steps,
                                                                        const float* __restrict__ ls,
                                                                        const float* __restrict__ le, VoxArgs va,
                                                                        float* __restrict__ cols,
@@ -52,12 +52,12 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) bisect_kernel(DevPlant
                                                                        float* __restrict__ dist) {
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
-  const WarpCtx<SM> w = warp_setup<SM>(p, smem4, &bar);
+  const WarpCtx<M> w = warp_setup<M>(p, smem4, &bar);
   if (!w.ok) return;
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
   for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < K; i += nw)
-    bisect_particle<SM>(p, w, i, dim, steps, ls, le, va, cols, proj, dist, lane);
+    bisect_particle<M>(p, w, i, dim, steps, ls, le, va, cols, proj, dist, lane);
 }
 
 // One block places up to max_faces faces (greedy, nearest collision first).
@@ -111,19 +111,15 @@ static bool point_in_set(const std::vector<float>& A, const std::vector<float>& 
 static csd_status_t launch_bisect(const csd_plant_s* p, int K, int dim, int steps, const float* ls, const float* le,
                                   const VoxArgs& va, float* cols, float* proj, float* dist, cudaStream_t st) {
   if (K <= 0) return CSD_OK;
-  const bool sm = statics_in_smem(p);
-  const size_t smem = (size_t)warp_floats(p->dp) * sizeof(float) * kWarpsPerBlock + (sm ? p->dp.static_bytes : 0);
-  int grid = 0;
-  csd_status_t s;
-  if (sm) {
-    if ((s = grid_for(bisect_kernel<true>, smem, K, &grid, kWarpsPerBlock))) return s;
-    bisect_kernel<true><<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, K, dim, steps, ls, le, va, cols, proj, dist);
-  } else {
-    if ((s = grid_for(bisect_kernel<false>, smem, K, &grid, kWarpsPerBlock))) return s;
-    bisect_kernel<false><<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, K, dim, steps, ls, le, va, cols, proj, dist);
-  }
-  CSD_CUDA_TRY(cudaGetLastError());
-  return CSD_OK;
+  return with_mode(plant_mode(p), [&](auto m) -> csd_status_t {
+    auto kernel = bisect_kernel<decltype(m)::value>;
+    const size_t smem = smem_bytes(p, kWarpsPerBlock);
+    int grid = 0;
+    if (csd_status_t s = grid_for(kernel, smem, K, &grid, kWarpsPerBlock)) return s;
+    kernel<<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, K, dim, steps, ls, le, va, cols, proj, dist);
+    CSD_CUDA_TRY(cudaGetLastError());
+    return CSD_OK;
+  });
 }
 
 }  // namespace csd

@@ -4,7 +4,7 @@
 #pragma once
 #include <cfloat>
 
-#include "check_core.cuh"
+#include "check_warp.cuh"
 #include "sampler_core.cuh"
 
 namespace csd {
@@ -63,8 +63,8 @@ static __device__ __forceinline__ void compact_block(const uint8_t* __restrict__
 // its projection and the bisection bounds; each step is a fused FK + check of
 // the midpoint. Dot products are accumulated in coordinate order with
 // fused multiply-adds (the order the CPU restatement uses).
-template <bool SM>
-static __device__ __forceinline__ void bisect_particle(const DevPlant& p, const WarpCtx<SM>& w, int i, int dim,
+template <int M>
+static __device__ __forceinline__ void bisect_particle(const DevPlant& p, const WarpCtx<M>& w, int i, int dim,
                                                        int steps, const float* __restrict__ ls,
                                                        const float* __restrict__ le, const VoxArgs& va,
                                                        float* __restrict__ cols, float* __restrict__ proj,
@@ -91,8 +91,7 @@ static __device__ __forceinline__ void bisect_particle(const DevPlant& p, const 
     __syncwarp();
     if (lane < dim) w.qs[lane] = mid;
     __syncwarp();
-    fk_warp(p, w.qs, w.X, lane);
-    const bool hit = check_config(p, w.stat, w.aabb, w.X, w.pose, lane, va);
+    const bool hit = check_warp<M>(p, w, lane, va);
     if (hit) {
       hi = mid;
       c = mid;

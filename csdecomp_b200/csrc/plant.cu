@@ -232,6 +232,7 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 csd_plant_s::~csd_plant_s() {
   if (blob) cudaFree(blob);
+  if (field_blob) cudaFree(field_blob);
 }
 
 using namespace csd;
@@ -418,6 +419,10 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
   std::vector<uint32_t> self_masks((size_t)T * nmsph, 0u);      // tile x moving-sphere partner
   std::vector<GenericPair> generic;
   std::vector<GenericPair> self_pairs;  // moving sphere x moving sphere
+  const int WS = (S + 31) / 32;
+  std::vector<uint32_t> world_bits((size_t)hp.moving.size() * WS, 0u);  // moving x static pairs
+  std::vector<uint32_t> moving_pairs;                                   // moving x moving, lower index first
+  const bool small = hp.moving.size() <= 0xffffu;
   int always = 0, tile_pairs = 0;
   auto ref = [&](int g) -> uint32_t {
     int m = hp.moving_of_geom[g];
@@ -432,6 +437,12 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
       const float* db = d->geom_dimensions + 3 * b;
       if (static_pair_hit(dgeom(d->geom_type[a], da, gX[a]), dgeom(d->geom_type[b], db, gX[b]))) always = 1;
       continue;
+    }
+    if (ma >= 0 && mb >= 0) {
+      if (small) moving_pairs.push_back((uint32_t)std::min(ma, mb) | (uint32_t)std::max(ma, mb) << 16);
+    } else {
+      const int st = hp.static_of_geom[ma >= 0 ? b : a];
+      world_bits[(size_t)std::max(ma, mb) * WS + (st >> 5)] |= 1u << (st & 31);
     }
     if ((ma >= 0 && mb < 0 && ma < nmsph) || (mb >= 0 && ma < 0 && mb < nmsph)) {
       int m = ma >= 0 ? ma : mb;
@@ -647,6 +658,41 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
   // reach some member, and the broad phase tests the others against no static
   // of the group (padded as the spheres; verdicts unchanged).
   std::vector<uint32_t> group_mask((size_t)std::max(NG, 0), 0u);
+  // box that every bounding sphere's points stay in (unbounded with a prismatic joint), and the statics' box
+  std::vector<double> reach_box{1e300, 1e300, 1e300, -1e300, -1e300, -1e300};
+  std::vector<double> static_box{1e300, 1e300, 1e300, -1e300, -1e300, -1e300};
+  std::vector<float> rounded((size_t)S * 8, 0.f);  // spheres and aligned boxes as rounded boxes
+  for (int st = 0; st < S; ++st) {
+    const float* W = hp.statics.data() + 16 * st;
+    const int ty = hp.static_type[st];
+    float* o = rounded.data() + 8 * st;
+    double c[3] = {W[0], W[1], W[2]}, e[3];
+    for (int r = 0; r < 3; ++r) {
+      if (ty == G_SPHERE) {
+        e[r] = W[3];
+      } else if (ty == G_CAPSULE) {
+        e[r] = std::fabs((double)W[4 + r]) * W[7] + W[3];
+      } else {
+        c[r] = e[r] = 0;
+        for (int a = 0; a < 3; ++a) {
+          c[r] += -(double)W[4 * a + 3] * W[4 * a + r];
+          e[r] += std::fabs((double)W[4 * a + r]) * W[12 + a];
+        }
+      }
+      static_box[r] = std::min(static_box[r], c[r] - e[r] * (1 + 1e-6) - 1e-4);
+      static_box[3 + r] = std::max(static_box[3 + r], c[r] + e[r] * (1 + 1e-6) + 1e-4);
+    }
+    if (ty == G_SPHERE) {
+      for (int r = 0; r < 4; ++r) o[r] = W[r];
+    } else if (st >= cls_begin[SC_ABOX] && st < cls_begin[SC_ABOX + 1]) {
+      for (int a = 0; a < 3; ++a) {
+        o[a] = -W[4 * a + 3];
+        o[4 + a] = W[12 + a];
+      }
+    } else {
+      o[7] = ty == G_BOX ? 1.f : 2.f;
+    }
+  }
   {
     std::vector<double> reach(NSL, 0.0), root((size_t)NSL * 3, 0.0);
     std::vector<char> bounded(NSL, 1);
@@ -661,6 +707,16 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
         for (int a = 0; a < 3; ++a) root[3 * k + a] = root[3 * f.parent + a];
         reach[k] = reach[f.parent] + tl;
         bounded[k] = bounded[f.parent] && f.type != J_PRISMATIC;
+      }
+    }
+    for (int k = 0; k < NSL; ++k) {
+      if (slot_bs[4 * k + 3] < 0.f) continue;
+      const double ck = std::sqrt((double)slot_bs[4 * k] * slot_bs[4 * k] + (double)slot_bs[4 * k + 1] * slot_bs[4 * k + 1] +
+                                  (double)slot_bs[4 * k + 2] * slot_bs[4 * k + 2]);
+      const double ext = bounded[k] ? (reach[k] + ck + slot_bs[4 * k + 3]) * (1 + 1e-6) + 1e-3 : 1e300;
+      for (int a = 0; a < 3; ++a) {
+        reach_box[a] = std::min(reach_box[a], root[3 * k + a] - ext);
+        reach_box[3 + a] = std::max(reach_box[3 + a], root[3 * k + a] + ext);
       }
     }
     for (int g = 0; g < NG; ++g)
@@ -791,6 +847,7 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
   dp.status = (int*)(base + o_status);
   dp.link_slot = (const int*)(base + o_ls);
   dp.link_fixed = (const float*)(base + o_lf);
+  if (csd_status_t s = build_field(h.get(), fk, moving_pairs, world_bits, rounded, static_box, reach_box)) return s;
   *out = h.release();
   return CSD_OK;
 }
