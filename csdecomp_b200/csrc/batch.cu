@@ -62,13 +62,15 @@ struct BatchIter {    // device-side iteration state
   int last_active;    // the count of the iteration that just finished
   int num_act;        // length of the active-slot list of iteration k
   int max_nf8;        // most faces of an active slot with dim <= 8
-  int max_nf16;       // most faces of an active slot with dim > 8
+  int max_nf16;       // most faces of an active slot with dim > 8 (of those not sampled from registers)
   int sample_next;    // work queues of the sampler, check and bisection launches: items claimed past the
   int check_next;     // first one per block (each zeroed before every launch that uses it)
   int bisect_next;
   int num_ord;        // active slots still checking in surrogate order (surrogate mode)
   int n_act;          // largest N_k of the active slots (work-item sizing)
   int num_fin;        // slots that finished in the last iteration, listed in BatchArgs::fin
+  int num_reg;        // the first num_reg listed slots are sampled from registers (region_in_regs)
+  int reg_next;       // their work queue
 };
 
 struct BatchArgs {
@@ -92,7 +94,7 @@ struct BatchArgs {
   float* fpool;
   uint8_t* bpool;
   BatchIter* it;
-  int* act;           // active-slot list of iteration k (slot indices, ascending)
+  int* act;           // active-slot list of iteration k (slot indices; ascending within each sampler's part)
   int* fin;           // slots that finished in the last iteration (the host harvests and refills them)
   // surrogate mode (mlp_wb null: off)
   const void* mlp_wb;
@@ -157,21 +159,25 @@ struct SampleStage {
 // alone and its arithmetic does not depend on G, so neither the order in
 // which blocks take items nor the variant changes a sample.
 template <int KP, int MINB>
-__global__ void __launch_bounds__(256, MINB) batch_sample_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(256, MINB) batch_sample_kernel(BatchArgs a, int from) {
   extern __shared__ __align__(16) float smf[];  // the face loop reads 16-byte vectors
   __shared__ GroupScratch gsa[kMaxWideGroups];
   const int N = a.it->n_act;  // items per slot are sized by the largest active N_k
-  const int64_t total = (int64_t)a.it->num_act * N;
+  // the listed slots past the first num_reg (from != 0: those run in batch_sample_regs_kernel) or all
+  const int skip = from ? a.it->num_reg : 0;
+  const int* act = a.act + skip;
+  const int num_act = a.it->num_act - skip;
+  const int64_t total = (int64_t)num_act * N;
   const int G0 = group_width(total, (int64_t)gridDim.x * (blockDim.x >> 5));
   int64_t c = total / (16 * (int64_t)gridDim.x);
   c = c < 32 ? 32 : c > 1024 ? 1024 : c;
   const int chunk = (int)(c / 32) * 32;
   const int ips = (N + chunk - 1) / chunk;
-  const int items = a.it->num_act * ips;  // at most slots * N / 32
+  const int items = num_act * ips;  // at most slots * N / 32
   constexpr int stage_floats = (int)(SampleStage<MINB>::bytes / sizeof(float));
   int staged = -1;
   for (int it = blockIdx.x; it < items;) {
-    const int slot = a.act[it / ips], first = (int)(it % ips) * chunk;
+    const int slot = act[it / ips], first = (int)(it % ips) * chunk;
     const SlotState& S = a.slots[slot];
     const int Ns = a.n_tab[S.k];
     if (first >= Ns) {  // past this slot's chains (uniform across the block)
@@ -207,6 +213,64 @@ __global__ void __launch_bounds__(256, MINB) batch_sample_kernel(BatchArgs a) {
     it = claim_item(&a.it->sample_next);
   }
 }
+
+// Chains of the first num_reg listed slots (all: of every listed slot), items
+// from the queue it->reg_next: the face pairs in registers
+// (sample_region_regs), or as batch_sample_kernel<8, 1> for a slot of another
+// size. One block per SM: four pairs of 14 coordinates and four chains' slacks
+// and dot products take 240 registers a thread.
+__global__ void __launch_bounds__(256, 1) batch_sample_regs_kernel(BatchArgs a, int all) {
+  extern __shared__ __align__(16) float smf[];
+  __shared__ GroupScratch gsa[kMaxWideGroups];
+  const int N = a.it->n_act, num = all ? a.it->num_act : a.it->num_reg;
+  int64_t c = (int64_t)num * N / (8 * (int64_t)gridDim.x);
+  c = c < 16 ? 16 : c > 1024 ? 1024 : c;
+  const int chunk = (int)(c / 16) * 16;
+  const int ips = (N + chunk - 1) / chunk;
+  const int items = num * ips;
+  const int G0 = group_width((int64_t)num * N, (int64_t)gridDim.x * (blockDim.x >> 5));
+  constexpr int stage_floats = (int)(SampleStage<1>::bytes / sizeof(float));
+  int staged = -1;
+  for (int it = blockIdx.x; it < items; it = claim_item(&a.it->reg_next)) {
+    const int slot = a.act[it / ips];
+    const SlotState& S = a.slots[slot];
+    const int first = (it % ips) * chunk, last = min(a.n_tab[S.k], first + chunk);
+    if (first >= last) continue;  // uniform across the block
+    const int dim = S.dim, P = (S.nf + 1) >> 1, rs = pair_stride(dim);
+    const float* rows = a.fpool + S.pr_off;
+    const float* ls = a.fpool + S.seg_off;
+    float* out = a.fpool + S.smp_off;
+    if (region_in_regs(dim, S.nf)) {
+      staged = -1;  // the buffer becomes scratch (claim_item's barriers are between its uses)
+      RegScratch* sc = reinterpret_cast<RegScratch*>(smf);
+      if (dim <= 14)
+        sample_region_regs<7>(rows, P, dim, ls, first, last, a.mixing, a.k0, a.k1, 0u, out, sc);
+      else
+        sample_region_regs<8>(rows, P, dim, ls, first, last, a.mixing, a.k0, a.k1, 0u, out, sc);
+      continue;
+    }
+    const int G = pair_group_width(G0, P, 8);
+    const bool fits = P * rs <= stage_floats;
+    if (fits && staged != slot) {
+      stage_pairs(rows, P, rs, smf);
+      __syncthreads();
+      staged = slot;
+    }
+    if (fits) {
+      if (dim <= 8)
+        sample_region<8, 8>(G, smf, P, dim, ls, first, last, a.mixing, a.k0, a.k1, 0u, out, gsa);
+      else
+        sample_region<16, 8>(G, smf, P, dim, ls, first, last, a.mixing, a.k0, a.k1, 0u, out, gsa);
+    } else {
+      if (dim <= 8)
+        sample_region<8, 8>(G, rows, P, dim, ls, first, last, a.mixing, a.k0, a.k1, 0u, out, gsa);
+      else
+        sample_region<16, 8>(G, rows, P, dim, ls, first, last, a.mixing, a.k0, a.k1, 0u, out, gsa);
+    }
+  }
+}
+constexpr size_t kRegSampleSmem = SampleStage<1>::bytes;
+static_assert(kRegSampleSmem >= 8 * sizeof(RegScratch), "scratch of eight groups");
 
 // Block per slot (slots slot0, slot0 + 1, ...): the face-pair rows of the
 // domain (start slacks at the slot's segment start).
@@ -351,13 +415,15 @@ __global__ void __launch_bounds__(1024) batch_faces_kernel(BatchArgs a) {
   if (threadIdx.x == 0 && !S.done) atomicAdd(&a.it->active, 1);
 }
 
-// One block: advances k and rebuilds the active-slot list (ascending).
+// One block: advances k and rebuilds the active-slot list: the slots sampled
+// from registers first, then the others, each part ascending.
 __global__ void __launch_bounds__(1024) batch_step_kernel(BatchArgs a) {
-  __shared__ int warp_n[32];
-  __shared__ int base, mf8, mf16, nord, nmax, nfin;
+  __shared__ int warp_n[2][32];
+  __shared__ int base[2], nreg, mf8, mf16, nord, nmax, nfin;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   if (tid == 0) {
-    base = 0;
+    base[0] = 0;
+    nreg = 0;
     mf8 = 0;
     mf16 = 0;
     nord = 0;
@@ -365,28 +431,41 @@ __global__ void __launch_bounds__(1024) batch_step_kernel(BatchArgs a) {
     nfin = 0;
   }
   __syncthreads();
+  for (int s = tid; s < a.num_slots; s += blockDim.x) {
+    SlotState& S = a.slots[s];
+    if (!S.done) {
+      S.k += 1;  // the slot finished its iteration and runs the next
+      const bool reg = region_in_regs(S.dim, S.nf);
+      if (reg)
+        atomicAdd(&nreg, 1);
+      else
+        atomicMax(S.dim <= 8 ? &mf8 : &mf16, S.nf);
+      atomicMax(&nmax, a.n_tab[min(S.k, a.max_iters - 1)]);
+      if (S.ord) atomicAdd(&nord, 1);
+    } else if (!S.harvested) {
+      S.harvested = 1;
+      a.fin[atomicAdd(&nfin, 1)] = s;  // finished this iteration: the host collects it
+    }
+  }
+  __syncthreads();
+  if (tid == 0) base[1] = nreg;  // part 0: from registers, part 1: the others
+  __syncthreads();
   for (int s0 = 0; s0 < a.num_slots; s0 += blockDim.x) {
     const int s = s0 + tid;
     const bool act = s < a.num_slots && !a.slots[s].done;
-    if (act) {
-      SlotState& S = a.slots[s];
-      S.k += 1;  // the slot finished its iteration and runs the next
-      atomicMax(S.dim <= 8 ? &mf8 : &mf16, S.nf);
-      atomicMax(&nmax, a.n_tab[min(S.k, a.max_iters - 1)]);
-      if (S.ord) atomicAdd(&nord, 1);
-    } else if (s < a.num_slots && !a.slots[s].harvested) {
-      a.slots[s].harvested = 1;
-      a.fin[atomicAdd(&nfin, 1)] = s;  // finished this iteration: the host collects it
+    const int part = act && !region_in_regs(a.slots[s].dim, a.slots[s].nf);
+    const unsigned m0 = __ballot_sync(0xffffffffu, act && part == 0), m1 = __ballot_sync(0xffffffffu, act && part == 1);
+    if (lane == 0) {
+      warp_n[0][warp] = __popc(m0);
+      warp_n[1][warp] = __popc(m1);
     }
-    const unsigned m = __ballot_sync(0xffffffffu, act);
-    if (lane == 0) warp_n[warp] = __popc(m);
     __syncthreads();
-    int off = base;
-    for (int w = 0; w < warp; ++w) off += warp_n[w];
-    if (act) a.act[off + __popc(m & ((1u << lane) - 1u))] = s;
+    int off = base[part];
+    for (int w = 0; w < warp; ++w) off += warp_n[part][w];
+    if (act) a.act[off + __popc((part ? m1 : m0) & ((1u << lane) - 1u))] = s;
     __syncthreads();
-    if (tid == 0)
-      for (int w = 0; w < nw; ++w) base += warp_n[w];
+    if (tid < 2)
+      for (int w = 0; w < nw; ++w) base[tid] += warp_n[tid][w];
     __syncthreads();
   }
   if (tid == 0) {
@@ -394,7 +473,8 @@ __global__ void __launch_bounds__(1024) batch_step_kernel(BatchArgs a) {
     it->last_active = it->active;
     it->active = 0;
     it->k += 1;
-    it->num_act = base;
+    it->num_act = base[1];
+    it->num_reg = nreg;
     it->max_nf8 = mf8;
     it->max_nf16 = mf16;
     it->num_ord = nord;
@@ -662,7 +742,7 @@ __global__ void __launch_bounds__(1024) batch_compact_sorted_kernel(BatchArgs a)
 // most (register-held slacks; wider groups for larger regions) and MINB
 // resident blocks per SM (register cap and staging buffer). Every variant
 // yields the same samples.
-using SampleFn = void (*)(BatchArgs);
+using SampleFn = void (*)(BatchArgs, int);
 struct SampleVariant {
   SampleFn fn;
   int kp, minb;
@@ -726,11 +806,16 @@ struct csd_batch_s {
   csd::DevBuf scores, order, status;
   std::vector<long long> job_configs;  // configurations checked per inflation of the last call
   std::vector<int> act_host;
-  cudaGraphExec_t graph = nullptr;
-  int graph_slots = -1, graph_cfg = -1, graph_variant = -1;
-  int graph_kernels = 0;        // kernel nodes of the captured iteration
+  // captured iterations by samplers launched (kSampleStaged | kSampleRegs)
+  struct IterationGraph {
+    cudaGraphExec_t exec = nullptr;
+    int slots = -1, cfg = -1, variant = -1;
+    const void* mlp = nullptr;
+    int kernels = 0;            // kernel nodes
+  } graphs[4];
+  cudaStream_t reg_stream = nullptr;  // the register sampler's branch of an iteration
+  cudaEvent_t fork = nullptr, join = nullptr;
   long long launches = 0;       // kernels launched by the last inflate
-  const void* graph_mlp = nullptr;
   cudaStream_t graph_stream = nullptr;
   csd::BatchIter* host_iter = nullptr;
   bool profile = false;         // launch stage by stage with events instead of the graph
@@ -744,7 +829,11 @@ struct csd_batch_s {
   ~csd_batch_s() {
     for (cudaEvent_t e : ev)
       if (e) cudaEventDestroy(e);
-    if (graph) cudaGraphExecDestroy(graph);
+    for (IterationGraph& g : graphs)
+      if (g.exec) cudaGraphExecDestroy(g.exec);
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    if (reg_stream) cudaStreamDestroy(reg_stream);
     if (graph_stream) cudaStreamDestroy(graph_stream);
     if (host_iter) cudaFreeHost(host_iter);
   }
@@ -795,17 +884,61 @@ void launch_check(const csd_batch_s* h, const BatchArgs& a, cudaStream_t s) {
   });
 }
 
+// The samplers of an iteration: batch_sample_kernel's variants and the
+// register sampler. Both, each on its own slots, where both have slots to fill
+// the GPU with; with few slots of one kind one launch takes all, the register
+// sampler from half of them on (it runs the other slots at one block per SM:
+// about 1.5 times their time, while the staged variants take about 1.7 times
+// the register sampler's on its own).
+enum : int { kSampleStaged = 1, kSampleRegs = 2 };
+constexpr int kSplitSlots = 8;
+int samplers_needed(const BatchIter& it) {
+  const int reg = it.num_reg, other = it.num_act - it.num_reg;
+  if (reg >= kSplitSlots && other >= kSplitSlots) return kSampleStaged | kSampleRegs;
+  return reg > 0 && reg >= other ? kSampleRegs : kSampleStaged;
+}
+
+void launch_staged_sampler(const csd_batch_s* h, int variant, int samplers, const BatchArgs& a, cudaStream_t s) {
+  const SampleVariant& v = kSampleVariants[variant];
+  v.fn<<<h->sample_grid[variant], 256, v.smem, s>>>(a, (samplers & kSampleRegs) ? 1 : 0);
+}
+
+// Two samplers run on parallel branches (the blocks of one fill what the
+// other's tail leaves idle). `launch`: which of the iteration's `samplers` to
+// launch. Returns the number of kernels launched.
+int launch_samplers(csd_batch_s* h, int samplers, int launch, const BatchArgs& a, cudaStream_t s) {
+  int n = 0;
+  const bool both = launch == (kSampleStaged | kSampleRegs);
+  if (launch & kSampleRegs) {
+    cudaMemsetAsync(&a.it->reg_next, 0, sizeof(int), s);
+    if (both) {
+      cudaEventRecord(h->fork, s);
+      cudaStreamWaitEvent(h->reg_stream, h->fork, 0);
+    }
+    batch_sample_regs_kernel<<<device_sm_count(), 256, kRegSampleSmem, both ? h->reg_stream : s>>>(
+        a, samplers == kSampleRegs ? 1 : 0);
+    ++n;
+  }
+  if (launch & kSampleStaged) {
+    cudaMemsetAsync(&a.it->sample_next, 0, sizeof(int), s);  // the work queue
+    launch_staged_sampler(h, h->run_variant, samplers, a, s);
+    ++n;
+  }
+  if (both) {
+    cudaEventRecord(h->join, h->reg_stream);
+    cudaStreamWaitEvent(s, h->join, 0);
+  }
+  return n;
+}
+
 // One iteration's launches on stream s. ev (kStages + 1 events) brackets the
-// stages for the profiling mode; skip_sample leaves out the sampler (the
-// autotuner has just run it).
+// stages for the profiling mode; `launch` says which of the iteration's samplers
+// to launch (the autotuner has just run the staged one).
 // Returns the number of kernels launched.
 int launch_iteration(csd_batch_s* h, int num_slots, const BatchArgs& a, cudaStream_t s, cudaEvent_t* ev,
-                     bool skip_sample = false) {
-  if (!skip_sample) cudaMemsetAsync(&a.it->sample_next, 0, sizeof(int), s);  // the sampler's work queue
+                     int samplers, int launch) {
   if (ev) cudaEventRecord(ev[0], s);
-  if (!skip_sample)
-    kSampleVariants[h->run_variant].fn<<<h->sample_grid[h->run_variant], 256, kSampleVariants[h->run_variant].smem,
-                                         s>>>(a);
+  const int sample_kernels = launch_samplers(h, samplers, launch, a, s);
   if (ev) cudaEventRecord(ev[1], s);
   if (a.mlp_wb) {
     batch_score_kernel<<<dim3((h->n_max + 127) / 128, num_slots), mlp::kThreads, mlp::kFwdSmem, s>>>(a);
@@ -843,37 +976,39 @@ int launch_iteration(csd_batch_s* h, int num_slots, const BatchArgs& a, cudaStre
   if (ev) cudaEventRecord(ev[7], s);
   batch_step_kernel<<<1, 1024, 0, s>>>(a);
   if (ev) cudaEventRecord(ev[8], s);
-  // sampler; score, sort, (check + tally) per round, compaction | check, compaction; bisect, faces, step
-  return (skip_sample ? 0 : 1) + (a.mlp_wb ? 3 + 2 * a.rounds : 2) + 3;
+  // samplers; score, sort, (check + tally) per round, compaction | check, compaction; bisect, faces, step
+  return sample_kernels + (a.mlp_wb ? 3 + 2 * a.rounds : 2) + 3;
 }
 
-csd_status_t build_graph(csd_batch_s* h, int num_slots, const BatchArgs& a) {
-  if (h->graph && h->graph_slots == num_slots && h->graph_cfg == a.cfg_max && h->graph_variant == h->run_variant &&
-      h->graph_mlp == a.mlp_wb)
+// The captured iteration with these samplers (captured again when a shape changed).
+csd_status_t build_graph(csd_batch_s* h, int num_slots, const BatchArgs& a, int samplers) {
+  csd_batch_s::IterationGraph& G = h->graphs[samplers];
+  if (G.exec && G.slots == num_slots && G.cfg == a.cfg_max && G.variant == h->run_variant && G.mlp == a.mlp_wb)
     return CSD_OK;
-  if (h->graph) {
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
+  if (G.exec) {
+    cudaGraphExecDestroy(G.exec);
+    G.exec = nullptr;
   }
   cudaStream_t s = h->graph_stream;
   cudaGraph_t g = nullptr;
   CSD_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  h->graph_kernels = launch_iteration(h, num_slots, a, s, nullptr);
+  G.kernels = launch_iteration(h, num_slots, a, s, nullptr, samplers, samplers);
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (e != cudaSuccess) {
     set_error(std::string("graph capture failed: ") + cudaGetErrorString(e));
     return CSD_ERR_CUDA;
   }
-  e = cudaGraphInstantiate(&h->graph, g, 0);
+  e = cudaGraphInstantiate(&G.exec, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) {
+    G.exec = nullptr;
     set_error(std::string("graph instantiation failed: ") + cudaGetErrorString(e));
     return CSD_ERR_CUDA;
   }
-  h->graph_slots = num_slots;
-  h->graph_cfg = a.cfg_max;
-  h->graph_variant = h->run_variant;
-  h->graph_mlp = a.mlp_wb;
+  G.slots = num_slots;
+  G.cfg = a.cfg_max;
+  G.variant = h->run_variant;
+  G.mlp = a.mlp_wb;
   return CSD_OK;
 }
 
@@ -953,6 +1088,7 @@ csd_status_t csd_batch_create(const csd_plant_t* plants, int32_t num_plants, int
                                                              kSampleVariants[v].smem));
     h->sample_grid[v] = device_sm_count() * std::max(1, per_sm);
   }
+  CSD_CUDA_TRY(raise_smem_limit(batch_sample_regs_kernel, kRegSampleSmem));
   // buffers
   const size_t per_slot_f = slot_floats(h.get());
   if ((s = h->plants_dev.reserve(dps.size() * sizeof(DevPlant))) || (s = h->slots_dev.reserve(max_slots * sizeof(SlotState))) ||
@@ -968,6 +1104,9 @@ csd_status_t csd_batch_create(const csd_plant_t* plants, int32_t num_plants, int
   CSD_CUDA_TRY(cudaMemcpy(t + K, h->m_tab.data(), K * 4, cudaMemcpyHostToDevice));
   CSD_CUDA_TRY(cudaMemcpy(t + 2 * K, h->thr_tab.data(), K * 4, cudaMemcpyHostToDevice));
   CSD_CUDA_TRY(cudaStreamCreateWithFlags(&h->graph_stream, cudaStreamNonBlocking));
+  CSD_CUDA_TRY(cudaStreamCreateWithFlags(&h->reg_stream, cudaStreamNonBlocking));
+  CSD_CUDA_TRY(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
+  CSD_CUDA_TRY(cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
   CSD_CUDA_TRY(cudaMallocHost((void**)&h->host_iter, sizeof(BatchIter)));
   *out = h.release();
   return CSD_OK;
@@ -1075,10 +1214,14 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
   BatchIter zero{};
   zero.num_act = ns;
   zero.n_act = h->n_tab[0];
-  *h->host_iter = zero;
-  CSD_CUDA_TRY(cudaMemcpyAsync(h->iter.ptr, h->host_iter, sizeof(BatchIter), cudaMemcpyHostToDevice, st));
+  // the slots whose domain is sampled from registers first, as the step kernel lists them
   h->act_host.resize(ns);
   for (int i = 0; i < ns; ++i) h->act_host[i] = i;
+  zero.num_reg = (int)(std::stable_partition(h->act_host.begin(), h->act_host.end(),
+                                             [&](int i) { return region_in_regs(slots[i].dim, slots[i].nf); }) -
+                       h->act_host.begin());
+  *h->host_iter = zero;
+  CSD_CUDA_TRY(cudaMemcpyAsync(h->iter.ptr, h->host_iter, sizeof(BatchIter), cudaMemcpyHostToDevice, st));
   CSD_CUDA_TRY(cudaMemcpyAsync(h->act.ptr, h->act_host.data(), (size_t)ns * 4, cudaMemcpyHostToDevice, st));
   BatchArgs a{};
   a.slots = h->slots_dev.as<SlotState>();
@@ -1122,7 +1265,6 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
   h->launches = 1;
   CSD_CUDA_TRY(cudaGetLastError());
   h->run_variant = h->sample_variant;
-  if ((s = build_graph(h, ns, a))) return s;
   // collected results: a finished slot's region, iteration count and configurations go to its inflation
   h->job_configs.assign(n, 0);
   std::vector<char> done_job(n, 0);
@@ -1160,6 +1302,7 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
   std::vector<int> fin;
   int active_now = ns;
   for (;;) {
+    const int samplers = samplers_needed(*h->host_iter);
     if (h->large_pending && h->tune_iters == 0) {
       // regions outgrew the tuned variant's staging for the first time: every sampler variant
       // on this iteration's inputs (the stage is idempotent), then the rest of the iteration;
@@ -1170,11 +1313,11 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
       for (int v = 0; v < kNumSampleVariants; ++v) {
         cudaMemsetAsync(&a.it->sample_next, 0, sizeof(int), st);
         cudaEventRecord(tev[2 * v], st);
-        kSampleVariants[v].fn<<<h->sample_grid[v], 256, kSampleVariants[v].smem, st>>>(a);
+        launch_staged_sampler(h, v, samplers, a, st);
         cudaEventRecord(tev[2 * v + 1], st);
         ++h->launches;
       }
-      h->launches += launch_iteration(h, ns, a, st, nullptr, true);
+      h->launches += launch_iteration(h, ns, a, st, nullptr, samplers, samplers & ~kSampleStaged);
       CSD_CUDA_TRY(cudaGetLastError());
       CSD_CUDA_TRY(cudaStreamSynchronize(st));
       int best = 0;
@@ -1188,7 +1331,6 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
       h->large_tuned = true;
       h->large_variant = best;
       h->run_variant = best;
-      if ((s = build_graph(h, ns, a))) return s;
       if (h->profile)
         CSD_CUDA_TRY(cudaMemcpyAsync(prof_slots.data(), h->slots_dev.ptr, ns * sizeof(SlotState),
                                      cudaMemcpyDeviceToHost, st));
@@ -1204,7 +1346,7 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
       for (int v = 0; v < kNumSampleVariants; ++v, ++j) {
         cudaMemsetAsync(&a.it->sample_next, 0, sizeof(int), st);
         cudaEventRecord(tev[2 * j], st);
-        kSampleVariants[v].fn<<<h->sample_grid[v], 256, kSampleVariants[v].smem, st>>>(a);
+        launch_staged_sampler(h, v, samplers, a, st);
         cudaEventRecord(tev[2 * j + 1], st);
         ++h->launches;
       }
@@ -1217,7 +1359,7 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
         cudaEventRecord(tev[2 * j + 1], st);
         ++h->launches;
       }
-      h->launches += launch_iteration(h, ns, a, st, nullptr, true);
+      h->launches += launch_iteration(h, ns, a, st, nullptr, samplers, samplers & ~kSampleStaged);
       CSD_CUDA_TRY(cudaGetLastError());
       CSD_CUDA_TRY(cudaStreamSynchronize(st));
       for (int q = 0; q < j; ++q) {
@@ -1239,11 +1381,9 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
         h->large_variant = variant_for(h, kSampleVariants[bs].f8 + 1, kSampleVariants[bs].f16 + 1);
         if (!a.mlp_wb) h->cfg_max = kCheckItemCaps[bc];
         a.cfg_max = h->cfg_max;
-        h->graph_slots = -1;  // recapture with the chosen shapes
-        if ((s = build_graph(h, ns, a))) return s;
       }
     } else if (h->profile) {
-      h->launches += launch_iteration(h, ns, a, st, h->ev);
+      h->launches += launch_iteration(h, ns, a, st, h->ev, samplers, samplers);
       CSD_CUDA_TRY(cudaGetLastError());
       CSD_CUDA_TRY(cudaEventSynchronize(h->ev[kStages]));
       for (int j = 0; j < kStages; ++j) {
@@ -1265,8 +1405,9 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
       CSD_CUDA_TRY(cudaMemcpyAsync(prof_slots.data(), h->slots_dev.ptr, ns * sizeof(SlotState),
                                    cudaMemcpyDeviceToHost, st));
     } else {
-      CSD_CUDA_TRY(cudaGraphLaunch(h->graph, st));
-      h->launches += h->graph_kernels;
+      if ((s = build_graph(h, ns, a, samplers))) return s;
+      CSD_CUDA_TRY(cudaGraphLaunch(h->graphs[samplers].exec, st));
+      h->launches += h->graphs[samplers].kernels;
     }
     CSD_CUDA_TRY(cudaMemcpyAsync(h->host_iter, h->iter.ptr, sizeof(BatchIter), cudaMemcpyDeviceToHost, st));
     CSD_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1316,7 +1457,6 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
     // same checks as a slot checking in sample order)
     if (a.mlp_wb && h->host_iter->num_ord == 0 && next_job >= n && h->tune_iters == 0) {
       a.mlp_wb = nullptr;
-      if ((s = build_graph(h, ns, a))) return s;
     }
     // a slot's region outgrew the staging buffer of the running variant: the first time, time
     // every variant on the next iteration; after that, continue with the fastest variant (by
@@ -1332,7 +1472,6 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
         if (v != h->run_variant) {
           h->run_variant = v;
           h->large_variant = v;
-          if ((s = build_graph(h, ns, a))) return s;
         }
       }
     }
@@ -1431,7 +1570,7 @@ csd_status_t csd_batch_set_surrogate_rounds(csd_batch_t h, int32_t rounds, int32
             "rounds must be in [1, 8] and the first round at least 32 samples");
   h->rounds = rounds;
   h->round_base = first_round;
-  h->graph_slots = -1;
+  for (csd_batch_s::IterationGraph& g : h->graphs) g.slots = -1;
   return CSD_OK;
 }
 

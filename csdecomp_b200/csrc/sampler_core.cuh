@@ -141,6 +141,81 @@ __device__ __forceinline__ void theta_bound(float s, float ad, float& tmin, floa
   tmax = ad > 0.0f ? fminf(tmax, q) : tmax;
 }
 
+// ---- theta bounds of a face pair without a division per face.
+//
+// Two correctly rounded quotients at once: reciprocal estimates (at most 1 ulp
+// off) and packed fused steps. y1 = y0 + y0 (1 - a y0) is the correctly
+// rounded reciprocal, q1 is within one ulp of s / a, and q1 + y1 (s - a q1)
+// then rounds as the quotient does (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1),
+// 1990, theorems 4 and 7), as long as nothing overflows or leaves the normal
+// range. na holds -a. tests/test_gpu_sampler_bounds.py compares it with the
+// IEEE division, the one significand that the theorem leaves out included.
+__device__ __forceinline__ float rcp_estimate(float a) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+  return y;
+}
+__device__ __forceinline__ uint64_t f2_quotient(uint64_t s, uint64_t na) {
+  float a0, a1;
+  f2_unpack(na, &a0, &a1);
+  const uint64_t y0 = f2_pack(rcp_estimate(-a0), rcp_estimate(-a1));
+  const uint64_t y1 = f2_fma(f2_fma(na, y0, f2_pack(1.f, 1.f)), y0, y0);
+  const uint64_t q0 = f2_mul(s, y0);
+  const uint64_t q1 = f2_fma(f2_fma(na, q0, s), y0, q0);
+  return f2_fma(f2_fma(na, q1, s), y1, q1);
+}
+
+// Running bounds as the bits of the quotients. While every slack is positive
+// a quotient has the sign of a . dir, and then theta_max, the least positive
+// quotient, is the least of the bit patterns as unsigned integers, and
+// theta_min, the negative quotient nearest to zero, the least as signed
+// integers: one three-way integer minimum each per face pair. (NaN and
+// infinite quotients, from a . dir = 0, lose against the initial
+// +-FLT_MAX as they do in theta_bound.) `slack` tracks the least slack the
+// same way.
+struct ThetaBits {
+  uint32_t hi;   // theta_max
+  int32_t lo;    // theta_min
+  int32_t slack;
+};
+__device__ __forceinline__ ThetaBits theta_bits_start() {
+  return {__float_as_uint(FLT_MAX), __float_as_int(-FLT_MAX), __float_as_int(FLT_MAX)};
+}
+__device__ __forceinline__ void theta_bits(ThetaBits& t, uint64_t s, uint64_t na) {
+  const uint64_t q = f2_quotient(s, na);
+  const int q0 = (int)(uint32_t)q, q1 = (int)(q >> 32);
+  t.hi = __vimin3_u32(t.hi, (uint32_t)q0, (uint32_t)q1);
+  t.lo = __vimin3_s32(t.lo, q0, q1);
+  t.slack = __vimin3_s32(t.slack, (int)(uint32_t)s, (int)(s >> 32));
+}
+// Where that holds: every slack at least kMinSlack (a start on a face has none:
+// such a lane takes theta_bound over its faces), and both bounds of the group
+// within [kMinTheta, kMaxTheta), so that the binding a . dir lies in
+// [2^-59, 2^126) and its quotient is exact (otherwise the group takes
+// theta_bound). A face whose a . dir is too small or too large for the packed
+// steps has a quotient outside that range, so it cannot bind unseen.
+//
+// The slow path over n face pairs copied to local memory, in a loop that is
+// not unrolled: the branch is next to never taken, and with the quotients of
+// every register-held pair written out there the fast path lost 40% to the
+// registers they took (42 -> 25 cycles per 32 pairs, register rows at 14
+// dimensions).
+__device__ __forceinline__ void theta_bounds_slow(const uint64_t* s, const uint64_t* na, int n, float& tmin,
+                                                  float& tmax) {
+#pragma unroll 1
+  for (int j = 0; j < n; ++j) {
+    float sa, sb, aa, ab;
+    f2_unpack(s[j], &sa, &sb);
+    f2_unpack(na[j], &aa, &ab);
+    theta_bound(sa, -aa, tmin, tmax);
+    theta_bound(sb, -ab, tmin, tmax);
+  }
+}
+constexpr float kMinSlack = 9.313225746154785e-10f;   // 2^-30
+constexpr float kMinTheta = 7.888609052210118e-31f;   // 2^-100
+constexpr float kMaxTheta = 536870912.f;              // 2^29
+
 // Steps whose draws a group computes at once (when its drawing lanes hold
 // that many steps' jobs).
 constexpr int kDrawSteps = 8;
@@ -148,11 +223,12 @@ constexpr int kDrawSteps = 8;
 // Shared scratch of a group wider than a warp (G = 64, 128, 256 lanes): the
 // directions and theta uniforms of a batch of drawn steps (coordinates 0..15,
 // the uniform at 16), double buffered by batch parity, and each warp's
-// partial theta bounds, double buffered by step parity (a warp cannot run two
-// steps, or two batches, ahead of the group's barriers).
+// partial theta bounds, double buffered by step parity (a warp cannot
+// run two steps, or two batches, ahead of the group's barriers). The
+// directions are stored negated (see run_chain_pairs).
 struct GroupScratch {
   float dir[2][kDrawSteps][17];
-  float red[2][8][2];
+  float red[3][8][2];  // by step parity; [2]: a step's second reduction
 };
 constexpr int kMaxWideGroups = 4;  // 256 threads / 64 lanes
 
@@ -181,8 +257,10 @@ __host__ __device__ __forceinline__ int pair_group_width(int g, int P, int KP) {
 // lane t JB + p / 2. The direction reaches the group by shuffles (G <= 32) or
 // through GroupScratch (wider groups, named barrier bar_id). The theta bounds
 // are max/min reductions, which do not depend on the order, so every chain
-// ends bit for bit where the oracle's serial chain ends whatever G. A chain
-// whose line search fails keeps stepping without moving (the group's lanes
+// ends bit for bit where the oracle's serial chain ends whatever G. Directions
+// are drawn negated, so that the dot products are the -(a . dir) that the
+// quotients' residuals and (with the sign taken into theta) the slack and
+// position updates want; negation is exact. A chain whose line search fails keeps stepping without moving (the group's lanes
 // stay convergent) and returns false.
 template <int MAXD, int G, int KP>
 __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, int P, int dim, int mixing,
@@ -198,14 +276,14 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
   // a lane past the last pair in round j holds a copy of pair P - 1 there: its work is the same
   // as that pair's owner's (so the group's lanes never diverge in the face loop) and a face seen
   // twice changes no theta bound
-  uint64_t s2[KP], a2[KP];
+  uint64_t s2[KP], na2[KP];  // na2: -(a . dir)
 #pragma unroll
   for (int j = 0; j < KP; ++j) {
     const int p = min(gl + G * j, P - 1);
     s2[j] = P > 0 ? *reinterpret_cast<const uint64_t*>(rows + (size_t)p * RS + 2 * MAXD) : 0ull;
-    a2[j] = 0ull;  // with nth = -0 the first update leaves every slack as it is
+    na2[j] = 0ull;  // with th = -0 the first update leaves every slack as it is
   }
-  float nth = -0.0f;
+  float th = -0.0f;
   bool ok = true;
   // this lane's block: pair 2 bq (c0a, c1a) and pair 2 bq + 1 (c0b, c1b); where a pair index
   // reaches npairs its c0 holds the theta uniform instead
@@ -227,10 +305,10 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
         sincos_2pi(u01_open1(w[1]), &sna, &csa);
         sincos_2pi(u01_open1(w[3]), &snb, &csb);
         const bool ga = 2 * bq < npairs, gb = 2 * bq + 1 < npairs;
-        c0a = ga ? __fmul_rn(rada, csa) : ua;
-        c1a = __fmul_rn(rada, sna);
-        c0b = gb ? __fmul_rn(radb, csb) : ub;
-        c1b = __fmul_rn(radb, snb);
+        c0a = ga ? -__fmul_rn(rada, csa) : ua;
+        c1a = -__fmul_rn(rada, sna);
+        c0b = gb ? -__fmul_rn(radb, csb) : ub;
+        c1b = -__fmul_rn(radb, snb);
       }
       if constexpr (G > 32) {
         if (gl < S * JB) {  // the first warp's lanes (S JB <= 32)
@@ -251,7 +329,7 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
       }
     }
     const int base = t * JB;  // lane of this step's block 0
-    uint64_t dd[MAXD];        // (dir_k, dir_k)
+    uint64_t dd[MAXD];        // (-dir_k, -dir_k)
     float ut;
     if constexpr (G <= 32) {
 #pragma unroll
@@ -273,13 +351,13 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
       }
       ut = db[16];
     }
-    float tmax = FLT_MAX, tmin = -FLT_MAX;
-    const uint64_t nth2 = f2_pack(nth, nth);
+    ThetaBits tb = theta_bits_start();
+    const uint64_t th2 = f2_pack(th, th);
 #pragma unroll
     for (int j = 0; j < KP; ++j) {
       if (G * j >= P) break;  // no lane of the group holds pair j (uniform across the group)
       const int p = min(gl + G * j, P - 1);
-      const uint64_t s = f2_fma(nth2, a2[j], s2[j]);  // the previous step's slack update
+      const uint64_t s = f2_fma(th2, na2[j], s2[j]);  // the previous step's slack update
       s2[j] = s;
       const ulonglong2* row = reinterpret_cast<const ulonglong2*>(rows + (size_t)p * RS);
       uint64_t acc = 0ull;
@@ -291,38 +369,55 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
           if (2 * q + 1 < dim) acc = f2_fma(v.y, dd[2 * q + 1], acc);
         }
       }
-      a2[j] = acc;
-      float sa, sb, aa, ab;
-      f2_unpack(s, &sa, &sb);
-      f2_unpack(acc, &aa, &ab);
-      theta_bound(sa, aa, tmin, tmax);
-      theta_bound(sb, ab, tmin, tmax);
+      na2[j] = acc;
+      theta_bits(tb, s, acc);
     }
-    if constexpr (G <= 32) {
+    float tmax, tmin;
+    for (int pass = 0;; ++pass) {
+      if (pass || tb.slack < __float_as_int(kMinSlack)) {  // this lane's faces one division each
+        tmax = FLT_MAX;
+        tmin = -FLT_MAX;
+        uint64_t ls[KP], ln[KP];
 #pragma unroll
-      for (int o = G / 2; o; o >>= 1) {
-        tmin = fmaxf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o, G));
-        tmax = fminf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o, G));
+        for (int j = 0; j < KP; ++j) {
+          ls[j] = s2[j];
+          ln[j] = na2[j];
+        }
+        theta_bounds_slow(ls, ln, min(KP, (P + G - 1) / G), tmin, tmax);
+      } else {
+        tmax = __uint_as_float(tb.hi);
+        tmin = __int_as_float(tb.lo);
       }
-    } else {
+      if constexpr (G <= 32) {
 #pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        tmin = fmaxf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
-        tmax = fminf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-      }
-      float(*red)[2] = gs->red[step & 1];
-      if ((gl & 31) == 0) {
-        red[gl >> 5][0] = tmin;
-        red[gl >> 5][1] = tmax;
-      }
-      group_bar(bar_id, G);
-      tmin = red[0][0];
-      tmax = red[0][1];
+        for (int o = G / 2; o; o >>= 1) {
+          tmin = fmaxf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o, G));
+          tmax = fminf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o, G));
+        }
+      } else {
 #pragma unroll
-      for (int w = 1; w < G / 32; ++w) {
-        tmin = fmaxf(tmin, red[w][0]);
-        tmax = fminf(tmax, red[w][1]);
+        for (int o = 16; o; o >>= 1) {
+          tmin = fmaxf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
+          tmax = fminf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+        }
+        float(*red)[2] = gs->red[pass ? 2 : step & 1];
+        if ((gl & 31) == 0) {
+          red[gl >> 5][0] = tmin;
+          red[gl >> 5][1] = tmax;
+        }
+        group_bar(bar_id, G);
+        tmin = red[0][0];
+        tmax = red[0][1];
+#pragma unroll
+        for (int w = 1; w < G / 32; ++w) {
+          tmin = fmaxf(tmin, red[w][0]);
+          tmax = fminf(tmax, red[w][1]);
+        }
       }
+      if (pass) break;
+      const bool in_range = tmax >= kMinTheta && tmax < kMaxTheta && -tmin >= kMinTheta && -tmin < kMaxTheta;
+      // uniform across the warp (G <= 32: its groups share the shuffles) or the group
+      if (G <= 32 ? __all_sync(0xffffffffu, in_range) : in_range) break;
     }
     if (isinf(tmax) || isinf(tmin) || tmax < tmin) ok = false;
     // this step's direction at the position coordinates the lane holds (coordinate k: block
@@ -340,15 +435,15 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
         dkl[r] = gs->dir[batch & 1][t][k];
       }
     }
-    nth = -0.0f;
+    th = -0.0f;
     if (ok) {
-      double th = __dadd_rn(__dmul_rn((double)ut, __dsub_rn(__dmul_rn(0.999999, (double)tmax), (double)tmin)),
+      const double td = __dadd_rn(__dmul_rn((double)ut, __dsub_rn(__dmul_rn(0.999999, (double)tmax), (double)tmin)),
                             (double)tmin);
-      const float theta = __double2float_rn(th);
+      const float theta = __double2float_rn(td);
 #pragma unroll
       for (int r = 0; r < XL; ++r)
-        if (gl + G * r < dim) xl[r] = __fmaf_rn(theta, dkl[r], xl[r]);
-      nth = -theta;
+        if (gl + G * r < dim) xl[r] = __fmaf_rn(-theta, dkl[r], xl[r]);
+      th = theta;
     }
     t = t + 1 == S ? 0 : t + 1;
   }
@@ -413,6 +508,239 @@ __device__ __forceinline__ void sample_region(int G, const float* __restrict__ r
       break;
     default:
       sample_chains_pairs<MAXD, 256, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
+      break;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Large regions above 8 dimensions: the face pairs stay in registers.
+//
+// run_chain_pairs reads every pair's coefficients from shared memory for every
+// chain and step: 7 16-byte loads per pair at 14 dimensions, 4 cycles of the
+// SM's shared-memory port each when 32 lanes read 32 rows. On regions of a few
+// hundred faces that port was 84% busy and the issue slots 47%: nothing else
+// could make it faster. Here a lane holds KR pairs' coefficients in registers
+// for all chains of a work item, and a group of W warps runs C chains side by
+// side; a step reads only the C directions (stored twice per coordinate, the
+// packed FMA's operand), the same address for all lanes. Per pair and chain
+// that is 7 / KR broadcast loads instead of 7 distinct ones.
+//
+// Per step: dot products, slack updates and quotient bounds (theta_bits) of
+// the lane's KR x C pairs; one integer warp minimum per bound and chain;
+// partials of the W warps through shared memory behind the group's barrier;
+// then every warp works out theta of the C chains (8 lanes each, which also
+// hold the chain's position). Same draws, same operations per face, order-free
+// minima: bit for bit the chains of run_chain_pairs.
+constexpr int kRegChains = 4;  // C: 8 lanes each in the theta phase
+constexpr int kRegSteps = 8;   // steps drawn at once
+// Row of the warp `wig` of group `gid`: rotated by group, so that the warps
+// with one row more than the others sit on different schedulers.
+__device__ __forceinline__ int reg_row(int wig, int gid, int W) { return (wig + gid) & (W - 1); }
+struct RegScratch {            // per group
+  float dir[2][kRegChains][kRegSteps][32];  // (-dir_k, -dir_k), by batch parity
+  float ut[2][kRegChains][kRegSteps];
+  float red[3][kRegChains][8][2];           // (theta_min, theta_max) per warp, by step parity; [2]: second pass
+};
+
+//
+// KR is the calling warp's own count: a region of R = ceil(P / 32) rows of 32
+// pairs gives warp r of the group rows r, r + W, ..., so the group's warps may
+// run different instantiations, which meet at the same barriers.
+template <int NQ, int KR>
+__device__ __forceinline__ void sample_chains_regs(const float* __restrict__ rows, int P, int dim,
+                                                   const float* __restrict__ start, int first, int last, int mixing,
+                                                   uint32_t k0, uint32_t k1, uint32_t stream, int W,
+                                                   float* __restrict__ out, RegScratch* scratch) {
+  constexpr int C = kRegChains, S = kRegSteps, RS = 2 * 16 + 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gid = warp / W, wig = warp - gid * W, ngroups = (int)(blockDim.x >> 5) / W;
+  const int gl = wig * 32 + lane, GL = 32 * W, bar_id = 1 + gid;
+  RegScratch& sc = scratch[gid];
+  const int npairs = (dim + 1) >> 1, JB = (npairs >> 1) + 1;
+  // this lane's pairs; past the last pair: copies of it (they bound what it bounds)
+  uint64_t a[KR][2 * NQ], s0[KR];
+  const int row0 = reg_row(wig, gid, W);
+#pragma unroll
+  for (int j = 0; j < KR; ++j) {
+    const float* r = rows + (size_t)min(32 * (row0 + W * j) + lane, P - 1) * RS;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(r + 4 * q);
+      a[j][2 * q] = v.x;
+      a[j][2 * q + 1] = v.y;
+    }
+    s0[j] = *reinterpret_cast<const uint64_t*>(r + 32);
+  }
+  // coordinates past dim have zero coefficients; their direction must only be finite
+  for (int i = gl; i < 2 * C * S * 32; i += GL) (&sc.dir[0][0][0][0])[i] = 0.f;
+  const int tc = lane >> 3, ti = lane & 7;  // theta phase: chain and coordinates ti, ti + 8
+  group_bar(bar_id, GL);
+  for (int c0 = first + gid * C; c0 < last; c0 += ngroups * C) {
+    uint64_t s2[C][KR], na2[C][KR];
+    float th[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      th[c] = -0.0f;
+#pragma unroll
+      for (int j = 0; j < KR; ++j) {
+        s2[c][j] = s0[j];
+        na2[c][j] = 0ull;
+      }
+    }
+    float x0 = ti < dim ? start[ti] : 0.f, x1 = ti + 8 < dim ? start[ti + 8] : 0.f;
+    bool ok = true;
+    int t = 0, par = 1;
+    for (int step = 0; step < mixing; ++step) {
+      if (t == 0) {
+        par ^= 1;
+        for (int job = gl; job < C * S * JB; job += GL) {
+          const int bq = job % JB, ct = job / JB, c = ct % C, tq = ct / C;
+          uint32_t w[4];
+          philox4x32_10((uint32_t)(step + tq), (uint32_t)min(c0 + c, last - 1), stream, (uint32_t)bq, k0, k1, w);
+          const float ua = u01_open0(w[0]), ub = u01_open0(w[2]);
+          const float rada = __fsqrt_rn(__fmul_rn(-2.0f, log_unit(ua)));
+          const float radb = __fsqrt_rn(__fmul_rn(-2.0f, log_unit(ub)));
+          float sna, csa, snb, csb;
+          sincos_2pi(u01_open1(w[1]), &sna, &csa);
+          sincos_2pi(u01_open1(w[3]), &snb, &csb);
+          float4* d = reinterpret_cast<float4*>(&sc.dir[par][c][tq][8 * bq]);
+          if (2 * bq < npairs) {
+            const float g0 = -__fmul_rn(rada, csa), g1 = -__fmul_rn(rada, sna);
+            d[0] = make_float4(g0, g0, g1, g1);
+          } else {
+            sc.ut[par][c][tq] = ua;
+          }
+          if (2 * bq + 1 < npairs) {
+            const float g0 = -__fmul_rn(radb, csb), g1 = -__fmul_rn(radb, snb);
+            d[1] = make_float4(g0, g0, g1, g1);
+          } else if (2 * bq + 1 == npairs) {
+            sc.ut[par][c][tq] = ub;
+          }
+        }
+        group_bar(bar_id, GL);
+      }
+      float(*red)[8][2] = sc.red[step & 1];
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const uint64_t th2 = f2_pack(th[c], th[c]);
+#pragma unroll
+        for (int j = 0; j < KR; ++j) s2[c][j] = f2_fma(th2, na2[c][j], s2[c][j]);
+      }
+      // coordinates outermost: C x KR independent dot products hide each other's latency
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const ulonglong2 dd = *reinterpret_cast<const ulonglong2*>(&sc.dir[par][c][t][4 * q]);
+#pragma unroll
+          for (int j = 0; j < KR; ++j) {
+            na2[c][j] = q == 0 ? f2_mul(a[j][0], dd.x) : f2_fma(a[j][2 * q], dd.x, na2[c][j]);
+            na2[c][j] = f2_fma(a[j][2 * q + 1], dd.y, na2[c][j]);
+          }
+        }
+      }
+      ThetaBits tb[C];
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        tb[c] = theta_bits_start();
+#pragma unroll
+        for (int j = 0; j < KR; ++j) theta_bits(tb[c], s2[c][j], na2[c][j]);
+      }
+      // a slack too small for the packed quotients: theta_max = 0 sends the group to the second pass
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        tb[c].hi = tb[c].slack < __float_as_int(kMinSlack) ? 0u : tb[c].hi;
+        tb[c].hi = __reduce_min_sync(0xffffffffu, tb[c].hi);
+        tb[c].lo = __reduce_min_sync(0xffffffffu, tb[c].lo);
+      }
+      if (lane == 0) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+          *reinterpret_cast<float2*>(red[c][wig]) = make_float2(__int_as_float(tb[c].lo), __uint_as_float(tb[c].hi));
+      }
+      float tmin, tmax;
+      for (int pass = 0;; ++pass) {
+        group_bar(bar_id, GL);
+        const float2 v = *reinterpret_cast<const float2*>(red[tc][min(ti, W - 1)]);
+        tmin = v.x;
+        tmax = v.y;
+#pragma unroll
+        for (int o = 4; o; o >>= 1) {
+          tmin = fmaxf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
+          tmax = fminf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+        }
+        const bool in_range = tmax >= kMinTheta && tmax < kMaxTheta && -tmin >= kMinTheta && -tmin < kMaxTheta;
+        if (pass || __all_sync(0xffffffffu, in_range)) break;  // the same in every warp of the group
+        red = sc.red[2];
+        uint64_t ls[C * KR], ln[C * KR];
+#pragma unroll
+        for (int i = 0; i < C * KR; ++i) {
+          ls[i] = s2[i / KR][i % KR];
+          ln[i] = na2[i / KR][i % KR];
+        }
+#pragma unroll 1
+        for (int c = 0; c < C; ++c) {
+          float lmax = FLT_MAX, lmin = -FLT_MAX;
+          theta_bounds_slow(ls + c * KR, ln + c * KR, KR, lmin, lmax);
+#pragma unroll
+          for (int o = 16; o; o >>= 1) {
+            lmin = fmaxf(lmin, __shfl_xor_sync(0xffffffffu, lmin, o));
+            lmax = fminf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+          }
+          if (lane == 0) *reinterpret_cast<float2*>(red[c][wig]) = make_float2(lmin, lmax);
+        }
+      }
+      if (isinf(tmax) || isinf(tmin) || tmax < tmin) ok = false;
+      float theta = -0.0f;
+      if (ok) {
+        const double ut = (double)sc.ut[par][tc][t];
+        theta = __double2float_rn(__dadd_rn(
+            __dmul_rn(ut, __dsub_rn(__dmul_rn(0.999999, (double)tmax), (double)tmin)), (double)tmin));
+        const float* d = sc.dir[par][tc][t];
+        x0 = ti < dim ? __fmaf_rn(-theta, d[2 * ti], x0) : x0;
+        x1 = ti + 8 < dim ? __fmaf_rn(-theta, d[2 * ti + 16], x1) : x1;
+      }
+#pragma unroll
+      for (int c = 0; c < C; ++c) th[c] = __shfl_sync(0xffffffffu, theta, 8 * c);
+      t = t + 1 == S ? 0 : t + 1;
+    }
+    const int chain = c0 + tc;
+    if (wig == 0 && chain < last) {
+      if (ti < dim) out[(int64_t)chain * dim + ti] = ok ? x0 : start[ti];
+      if (ti + 8 < dim) out[(int64_t)chain * dim + ti + 8] = ok ? x1 : start[ti + 8];
+    }
+    // the next chains' draws overwrite what this warp may be ahead of: dir[par] (read by slower warps)
+    group_bar(bar_id, GL);
+  }
+}
+
+// Regions sampled from registers: more than 8 dimensions and 65 to 1,024 face
+// pairs, two to four of them per lane. SM cycles per chain and step at 14
+// dimensions, from registers against run_chain_pairs' best (16 pairs per lane,
+// 2 blocks per SM): 93 / 119 with 75 pairs, 112 / 175 with 125, 204 / 340 with
+// 250, 391 / 674 with 500. Up to 64 pairs run_chain_pairs splits a warp over
+// four chains and wins; beyond 1,024 the pairs do not fit a block's registers.
+constexpr int kRegMinPairs = 65, kRegMaxPairs = 1024;
+__host__ __device__ __forceinline__ bool region_in_regs(int dim, int faces) {
+  const int P = (faces + 1) >> 1;
+  return dim > 8 && P >= kRegMinPairs && P <= kRegMaxPairs;
+}
+template <int NQ>
+__device__ __forceinline__ void sample_region_regs(const float* __restrict__ rows, int P, int dim,
+                                                   const float* __restrict__ start, int first, int last, int mixing,
+                                                   uint32_t k0, uint32_t k1, uint32_t stream,
+                                                   float* __restrict__ out, RegScratch* scratch) {
+  const int R = (P + 31) >> 5, W = R <= 4 ? 1 : R <= 8 ? 2 : R <= 16 ? 4 : 8;
+  const int warp = threadIdx.x >> 5, gid = warp / W;
+  switch ((R - reg_row(warp - gid * W, gid, W) + W - 1) / W) {  // this warp's rows
+    case 2:
+      sample_chains_regs<NQ, 2>(rows, P, dim, start, first, last, mixing, k0, k1, stream, W, out, scratch);
+      break;
+    case 3:
+      sample_chains_regs<NQ, 3>(rows, P, dim, start, first, last, mixing, k0, k1, stream, W, out, scratch);
+      break;
+    default:
+      sample_chains_regs<NQ, 4>(rows, P, dim, start, first, last, mixing, k0, k1, stream, W, out, scratch);
       break;
   }
 }
