@@ -41,7 +41,10 @@ struct FkJoint {
   int type, parent, child, qidx;
   float P[9], S[9], T[9];
   float t[3], v[3];
-  float pad[3];
+  // fk_kernel: where a transform that a later, not the next, joint hangs off is kept (-1: nowhere), and where
+  // this joint's parent transform is (-1: it is the joint before)
+  int save, from;
+  float pad;
 };
 static_assert(sizeof(FkJoint) == 160, "FkJoint is 10 float4");
 
@@ -140,6 +143,7 @@ struct DevPlant {
   int pose_words;        // words of moving world poses per configuration
   int always_colliding;  // a static-static pair collides
   int num_links;         // all links of the reference tree (FK output)
+  int num_saved;         // transforms fk_kernel keeps (FkJoint::save)
   int static_bytes;      // bytes of statics + aabb staged in shared memory (multiple of 16)
   int dense_spheres;     // every tile pairs every lane with every static sphere and aligned box
   int cull;              // link-level broad phase on (slot and static bounding spheres)

@@ -315,6 +315,15 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
     X[cl] = ident();
   }
 
+  int num_saved = 0;
+  for (FkJoint& f : fk) f.save = f.from = -1;
+  for (size_t j = 0; j < fk.size(); ++j) {
+    if (fk[j].parent < 0 || fk[j].parent == (int)j - 1) continue;
+    FkJoint& par = fk[fk[j].parent];
+    if (par.save < 0) par.save = num_saved++;
+    fk[j].from = par.save;
+  }
+
   // ---- geometries
   std::unique_ptr<csd_plant_s> h(new csd_plant_s());
   cudaGetDevice(&h->device);
@@ -830,6 +839,7 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
     dp.dense_spheres = dense;
   }
   dp.num_links = L;
+  dp.num_saved = num_saved;
   dp.cull = NSL >= 1 && NSL <= 32 && S <= 32 * 32;
   h->cull_eligible = dp.cull != 0;
   dp.slot_bs = (const float4*)(base + o_slb);
