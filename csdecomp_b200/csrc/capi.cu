@@ -365,7 +365,7 @@ csd_status_t csd_uniform_sample_hpolyhedra(const float* A, const float* b, const
       CSD_CUDA_TRY(cudaMallocAsync((void**)&nf, sizeof(int), st));
       CSD_CUDA_TRY(cudaMemsetAsync(nf, 0, sizeof(int), st));
     }
-    csd_status_t s = launch_hit_and_run(A, b, face_off, P, dim, starts, S, mixing, seed, 0u, 0, samples, nf, nullptr, st);
+    csd_status_t s = launch_hit_and_run(A, b, face_off, P, dim, starts, S, mixing, seed, samples, nf, st);
     if (num_failed) {
       if (!s) {
         cudaMemcpyAsync(num_failed, nf, sizeof(int), cudaMemcpyDeviceToHost, st);
@@ -415,7 +415,7 @@ csd_status_t csd_uniform_sample_hpolyhedra(const float* A, const float* b, const
   if (!s && cudaMemsetAsync(pnf, 0, sizeof(int), st) != cudaSuccess) s = CSD_ERR_CUDA;
   if (!s)
     s = launch_hit_and_run((const float*)pA, (const float*)pb, (const int32_t*)po, P, dim, (const float*)ps, S, mixing,
-                           seed, 0u, 0, (float*)pout, pnf, nullptr, st);
+                           seed, (float*)pout, pnf, st);
   int nf = 0;
   if (!s && (cudaMemcpyAsync(samples, pout, bout, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
              cudaMemcpyAsync(&nf, pnf, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

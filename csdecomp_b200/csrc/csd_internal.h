@@ -147,9 +147,8 @@ csd_status_t launch_check_edges_ranked(const csd_plant_s* p, const float* s0, co
                                        int64_t* pts, unsigned int* counter, cudaStream_t st);
 // sampler.cu
 csd_status_t launch_hit_and_run(const float* A, const float* b, const int32_t* face_off, int num_poly, int dim,
-                                const float* starts, int samples_per_poly, int mixing, uint64_t seed,
-                                uint32_t stream_base, int fail_keep, float* out, int* num_failed,
-                                const int* num_faces_dev, cudaStream_t st);
+                                const float* starts, int samples_per_poly, int mixing, uint64_t seed, float* out,
+                                int* num_failed, cudaStream_t st);
 // EI-ZO sampler over one region stored as face-pair rows (sampler_core.cuh,
 // pair_stride(dim) floats per row, start slacks at `start`); the face count is
 // read on the device. A failed chain keeps its start point.

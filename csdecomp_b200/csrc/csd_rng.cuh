@@ -98,36 +98,8 @@ __device__ __forceinline__ void sincos_2pi(float v, float* sn, float* cs) {
   *cs = ((qd + 1) & 2) ? -cc : cc;
 }
 
-// Direction (dim Gaussians) and the theta uniform of one mixing step.
-// Gaussian pair g uses words 2g (radius) and 2g+1 (angle); the theta uniform
-// is word 2*ceil(dim/2). Words 4k..4k+3 come from Philox block k.
-template <int MAXD>
-__device__ __forceinline__ void step_draws(uint32_t k0, uint32_t k1, uint32_t chain, uint32_t stream, uint32_t step,
-                                           int dim, float* dir, float* u_theta) {
-  const int npairs = (dim + 1) >> 1;
-  uint32_t w[4];
-  int have_block = -1;
-#pragma unroll
-  for (int g = 0; g < (MAXD + 1) / 2; ++g) {
-    if (g < npairs) {
-      int blk = (2 * g) >> 2;
-      if (blk != have_block) {
-        philox4x32_10(step, chain, stream, (uint32_t)blk, k0, k1, w);
-        have_block = blk;
-      }
-      float u = u01_open0(w[(2 * g) & 3]);
-      float v = u01_open1(w[(2 * g + 1) & 3]);
-      float rad = __fsqrt_rn(__fmul_rn(-2.0f, log_unit(u)));
-      float sn, cs;
-      sincos_2pi(v, &sn, &cs);
-      dir[2 * g] = __fmul_rn(rad, cs);
-      if (2 * g + 1 < MAXD) dir[2 * g + 1] = __fmul_rn(rad, sn);
-    }
-  }
-  int tw = 2 * npairs;
-  int blk = tw >> 2;
-  if (blk != have_block) philox4x32_10(step, chain, stream, (uint32_t)blk, k0, k1, w);
-  *u_theta = u01_open0(w[tw & 3]);
-}
+// One mixing step draws words 0 .. 2 ceil(dim/2): Gaussian pair g uses words 2g
+// (radius) and 2g + 1 (angle), the theta uniform is word 2 ceil(dim/2); words
+// 4k .. 4k + 3 come from Philox block k.
 
 }  // namespace csd

@@ -4,14 +4,14 @@
 // cuda_hit_and_run_sampling.cu:18-119: a Gaussian direction per mixing step,
 // slack b - A x and A dir per face, theta interval from the sign of (A dir)_i,
 // theta = u * (0.999999 * theta_max - theta_min) + theta_min (:106-107).
-// Same chain structure here; the face loop reads A and b with warp-uniform
-// addresses (every thread of a polytope walks the same face at the same time,
-// so each load is one broadcast transaction), keeps the chain state in
-// registers (the reference keeps two float[4000] arrays per thread in local
-// memory) and draws from the counter-based stream of csd_rng.cuh.
+// Same chain here with 8 to 32 lanes on it and the draws of csd_rng.cuh. A
+// thread per chain filled the GPU only from some 100,000 chains on: 16 regions
+// x 1,000 samples ran 500 warps, each a serial walk over the faces, 591 us
+// against 127 us here.
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
+#include <type_traits>
 
 #include "csd_internal.h"
 #include "csd_rng.cuh"
@@ -19,31 +19,158 @@
 
 namespace csd {
 
-template <int MAXD>
-__global__ void __launch_bounds__(128) hit_and_run_kernel(const float* __restrict__ A, const float* __restrict__ b,
-                                                          const int32_t* __restrict__ face_off,
-                                                          const int* __restrict__ num_faces_dev, int num_poly,
-                                                          int dim, const float* __restrict__ starts, int S,
-                                                          int mixing, uint32_t k0, uint32_t k1,
-                                                          uint32_t stream_base, int fail_keep,
-                                                          float* __restrict__ out, int* num_failed) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)num_poly * S) return;
-  const int poly = (int)(i / S);
-  const int s = (int)(i % S);
-  const int f0 = face_off ? face_off[poly] : 0;
-  const int F = face_off ? face_off[poly + 1] - f0 : *num_faces_dev;
-  float x[MAXD];
+// Chains of num_poly polytopes, G lanes each; block = `chunk` chains of one
+// polytope (cpp chunks per polytope), whose faces it stages as face-pair rows
+// with the offsets b where the EI-ZO rows have start slacks. A lane walks
+// pairs gl, gl + G, ...: both dot products (b - A x and A dir are recomputed
+// every step) as packed FMAs in the serial chain's order, the quotients packed
+// (theta_bits); every lane carries the whole position. Polytopes whose rows do
+// not fit the staging buffer are read face by face from global memory. Same
+// draws and operations per face as run_chain, and order-free bounds: the
+// chain is the serial chain's bit for bit.
+constexpr size_t kUniformStageBytes = 48 * 1024;
+// Floats of a row: coefficients, offsets, padded so that 8 consecutive rows fall on different banks.
+__host__ __device__ constexpr int uniform_stride(int nq) { return nq == 7 ? 36 : 4 * nq + 4; }
+
+template <int NQ, int G>  // NQ coordinate pairs (dim rounded up)
+__global__ void __launch_bounds__(256, NQ <= 4 ? 4 : 2)
+    hit_and_run_kernel(const float* __restrict__ A, const float* __restrict__ b, const int32_t* __restrict__ face_off,
+                       int dim, const float* __restrict__ starts, int S, int mixing, uint32_t k0, uint32_t k1,
+                       float* __restrict__ out, int* num_failed, int chunk, int cpp) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int MAXD = 2 * NQ, RS = uniform_stride(NQ);
+  const int poly = blockIdx.x / cpp, first = (blockIdx.x % cpp) * chunk, last = min(S, first + chunk);
+  const int f0 = face_off[poly], F = face_off[poly + 1] - f0, P = (F + 1) >> 1;
+  const float* Ap = A + (int64_t)f0 * dim;
+  const float* bp = b + f0;
+  const bool staged = (size_t)P * RS * sizeof(float) <= kUniformStageBytes;
+  if (staged) {
+    for (int i = threadIdx.x; i < 2 * P * MAXD; i += blockDim.x) {
+      const int p = i / (2 * MAXD), k = (i >> 1) % MAXD, f = min(2 * p + (i & 1), F - 1);  // an odd count repeats its last face
+      sm[p * RS + 2 * k + (i & 1)] = k < dim ? Ap[(int64_t)f * dim + k] : 0.f;
+    }
+    for (int i = threadIdx.x; i < 2 * P; i += blockDim.x) sm[(i >> 1) * RS + 2 * MAXD + (i & 1)] = bp[min(i, F - 1)];
+    __syncthreads();
+  }
+  const int gl = threadIdx.x & (G - 1), ngroups = blockDim.x / G;
+  const int npairs = (dim + 1) >> 1, JB = (npairs >> 1) + 1;
+  const int steps = min(kDrawSteps, G / JB), tq = gl / JB, bq = gl - tq * JB;  // draws as run_chain_pairs
+  const uint32_t stream = (uint32_t)poly;
+  for (int c0 = first; c0 < last; c0 += ngroups) {
+    const int mine = c0 + threadIdx.x / G, chain = min(mine, last - 1);
+    uint64_t xx[MAXD], dd[MAXD];  // (x_k, x_k), (-dir_k, -dir_k)
 #pragma unroll
-  for (int k = 0; k < MAXD; ++k) x[k] = k < dim ? starts[(int64_t)poly * dim + k] : 0.f;
-  const bool ok = run_chain<MAXD>(A + (int64_t)f0 * dim, b + f0, F, dim, mixing, k0, k1, (uint32_t)s,
-                                  stream_base + (uint32_t)poly, x);
-  if (!ok && num_failed) atomicAdd(num_failed, 1);
-  // a chain whose line search fails writes NaN, or (fail_keep) its start point
-  float* dst = out + i * dim;
+    for (int k = 0; k < MAXD; ++k) {
+      const float x = k < dim ? starts[(int64_t)poly * dim + k] : 0.f;
+      xx[k] = f2_pack(x, x);
+    }
+    bool ok = true;
+    float c0a = 0.f, c1a = 0.f, c0b = 0.f, c1b = 0.f;
+    int t = 0;
+    for (int step = 0; step < mixing; ++step) {
+      if (t == 0) {
+        uint32_t w[4];
+        philox4x32_10((uint32_t)(step + tq), (uint32_t)chain, stream, (uint32_t)bq, k0, k1, w);
+        const float ua = u01_open0(w[0]), ub = u01_open0(w[2]);
+        const float rada = __fsqrt_rn(__fmul_rn(-2.0f, log_unit(ua)));
+        const float radb = __fsqrt_rn(__fmul_rn(-2.0f, log_unit(ub)));
+        float sna, csa, snb, csb;
+        sincos_2pi(u01_open1(w[1]), &sna, &csa);
+        sincos_2pi(u01_open1(w[3]), &snb, &csb);
+        c0a = 2 * bq < npairs ? -__fmul_rn(rada, csa) : ua;
+        c1a = -__fmul_rn(rada, sna);
+        c0b = 2 * bq + 1 < npairs ? -__fmul_rn(radb, csb) : ub;
+        c1b = -__fmul_rn(radb, snb);
+      }
+      const int base = t * JB;
 #pragma unroll
-  for (int k = 0; k < MAXD; ++k)
-    if (k < dim) dst[k] = ok ? x[k] : fail_keep ? starts[(int64_t)poly * dim + k] : __int_as_float(0x7fc00000);
+      for (int k = 0; k < MAXD; ++k) {
+        const float v = ((k >> 1) & 1) ? ((k & 1) ? c1b : c0b) : ((k & 1) ? c1a : c0a);
+        const float dk = __shfl_sync(0xffffffffu, v, base + (k >> 2), G);
+        dd[k] = f2_pack(dk, dk);
+      }
+      const float ut = __shfl_sync(0xffffffffu, (npairs & 1) ? c0b : c0a, base + (npairs >> 1), G);
+      // pairs gl, gl + G, ... (staged): slacks and -(a . dir) of pair p
+      auto pair = [&](int p, uint64_t& s, uint64_t& na) {
+        const ulonglong2* row = reinterpret_cast<const ulonglong2*>(sm + p * RS);
+        uint64_t ax = 0ull;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {  // coefficients past dim are zero
+          const ulonglong2 v = row[q];
+          ax = q == 0 ? f2_mul(v.x, xx[0]) : f2_fma(v.x, xx[2 * q], ax);
+          na = q == 0 ? f2_mul(v.x, dd[0]) : f2_fma(v.x, dd[2 * q], na);
+          ax = f2_fma(v.y, xx[2 * q + 1], ax);
+          na = f2_fma(v.y, dd[2 * q + 1], na);
+        }
+        s = f2_sub(*reinterpret_cast<const uint64_t*>(sm + p * RS + 2 * MAXD), ax);
+      };
+      float tmax = FLT_MAX, tmin = -FLT_MAX;
+      for (int pass = staged ? 0 : 1;; ++pass) {
+        if (pass == 0) {
+          ThetaBits tb = theta_bits_start();
+          for (int p = gl; p < P; p += G) {
+            uint64_t s, na;
+            pair(p, s, na);
+            theta_bits(tb, s, na);
+          }
+          // a slack too small for the packed quotients: theta_max = 0 asks for the second pass
+          tmax = tb.slack < __float_as_int(kMinSlack) ? 0.f : __uint_as_float(tb.hi);
+          tmin = __int_as_float(tb.lo);
+        } else if (staged) {
+          tmax = FLT_MAX;
+          tmin = -FLT_MAX;
+          for (int p = gl; p < P; p += G) {
+            uint64_t s, na;
+            pair(p, s, na);
+            theta_bounds_slow(&s, &na, 1, tmin, tmax);
+          }
+        } else {
+          for (int f = gl; f < F; f += G) {
+            const float* a = Ap + (int64_t)f * dim;
+            float x0, d0, hi;
+            f2_unpack(xx[0], &x0, &hi);
+            f2_unpack(dd[0], &d0, &hi);
+            float ax = __fmul_rn(a[0], x0), na = __fmul_rn(a[0], d0);
+#pragma unroll
+            for (int k = 1; k < MAXD; ++k)
+              if (k < dim) {
+                f2_unpack(xx[k], &x0, &hi);
+                f2_unpack(dd[k], &d0, &hi);
+                ax = __fmaf_rn(a[k], x0, ax);
+                na = __fmaf_rn(a[k], d0, na);
+              }
+            theta_bound(__fsub_rn(bp[f], ax), -na, tmin, tmax);
+          }
+        }
+#pragma unroll
+        for (int o = G / 2; o; o >>= 1) {
+          tmin = fmaxf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o, G));
+          tmax = fminf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o, G));
+        }
+        const bool in_range = tmax >= kMinTheta && tmax < kMaxTheta && -tmin >= kMinTheta && -tmin < kMaxTheta;
+        if (pass || __all_sync(0xffffffffu, in_range)) break;  // uniform: the warp's groups share the shuffles
+      }
+      if (isinf(tmax) || isinf(tmin) || tmax < tmin) ok = false;
+      if (ok) {
+        const double th = __dadd_rn(__dmul_rn((double)ut, __dsub_rn(__dmul_rn(0.999999, (double)tmax), (double)tmin)),
+                                    (double)tmin);
+        const float nth = -__double2float_rn(th);
+        const uint64_t nth2 = f2_pack(nth, nth);
+#pragma unroll
+        for (int k = 0; k < MAXD; ++k)
+          if (k < dim) xx[k] = f2_fma(nth2, dd[k], xx[k]);
+      }
+      t = t + 1 == steps ? 0 : t + 1;
+    }
+    if (mine < last && gl == 0) {
+      if (!ok && num_failed) atomicAdd(num_failed, 1);
+      // a chain whose line search fails writes NaN
+      float* dst = out + ((int64_t)poly * S + chain) * dim;
+#pragma unroll
+      for (int k = 0; k < MAXD; ++k)
+        if (k < dim) dst[k] = ok ? __uint_as_float((uint32_t)xx[k]) : __int_as_float(0x7fc00000);
+    }
+  }
 }
 
 // EI-ZO sampler over one region (the single inflation and the
@@ -123,29 +250,39 @@ csd_status_t launch_put_faces(const float* A, const float* b, int F, int dim, co
 }
 
 csd_status_t launch_hit_and_run(const float* A, const float* b, const int32_t* face_off, int num_poly, int dim,
-                                const float* starts, int S, int mixing, uint64_t seed, uint32_t stream_base,
-                                int fail_keep, float* out, int* num_failed, const int* num_faces_dev,
+                                const float* starts, int S, int mixing, uint64_t seed, float* out, int* num_failed,
                                 cudaStream_t st) {
   const int64_t total = (int64_t)num_poly * S;
   if (total <= 0) return CSD_OK;
   CSD_CHECK(dim >= 1 && dim <= kMaxDim, CSD_ERR_DIMENSION, "dimension must be in [1, 16]");
-  const int threads = 128;
-  const int64_t blocks = (total + threads - 1) / threads;
+  // 8 lanes per chain once that gives every SM 16 warps, wider groups for fewer chains
+  const int64_t warps = (int64_t)device_sm_count() * 16;
+  const int G = total * 8 / 32 >= warps ? 8 : total * 16 / 32 >= warps ? 16 : 32;
+  const int groups = 256 / G;
+  // a block runs several rounds of chains only when there are blocks to spare (its staging is then shared)
+  const int64_t rounds = std::max<int64_t>(1, std::min<int64_t>(16, total / (groups * 4 * (int64_t)device_sm_count())));
+  const int chunk = (int)std::min<int64_t>(groups * rounds, ((int64_t)S + groups - 1) / groups * groups);
+  const int cpp = (S + chunk - 1) / chunk;
+  const int64_t blocks = (int64_t)num_poly * cpp;
   CSD_CHECK(blocks < (1ll << 31), CSD_ERR_CAPACITY, "too many samples");
-  uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-#define CSD_HR(MD)                                                                                         \
-  hit_and_run_kernel<MD><<<(unsigned)blocks, threads, 0, st>>>(A, b, face_off, num_faces_dev, num_poly, dim, \
-                                                               starts, S, mixing, k0, k1, stream_base,     \
-                                                               fail_keep, out, num_failed)
-  if (dim <= 2)
-    CSD_HR(2);
-  else if (dim <= 4)
-    CSD_HR(4);
+  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
+  auto launch = [&](auto kernel) {
+    kernel<<<(unsigned)blocks, 256, kUniformStageBytes, st>>>(A, b, face_off, dim, starts, S, mixing, k0, k1, out,
+                                                              num_failed, chunk, cpp);
+  };
+  auto by_width = [&](auto nq) {
+    constexpr int NQ = decltype(nq)::value;
+    G == 8 ? launch(hit_and_run_kernel<NQ, 8>) : G == 16 ? launch(hit_and_run_kernel<NQ, 16>)
+                                                         : launch(hit_and_run_kernel<NQ, 32>);
+  };
+  if (dim <= 4)
+    by_width(std::integral_constant<int, 2>());
   else if (dim <= 8)
-    CSD_HR(8);
+    by_width(std::integral_constant<int, 4>());
+  else if (dim <= 14)
+    by_width(std::integral_constant<int, 7>());
   else
-    CSD_HR(16);
-#undef CSD_HR
+    by_width(std::integral_constant<int, 8>());
   CSD_CUDA_TRY(cudaGetLastError());
   return CSD_OK;
 }

@@ -7,48 +7,6 @@
 
 namespace csd {
 
-// One hit-and-run chain (cuda_hit_and_run_sampling.cu:57-118): returns false
-// if a line search found an empty theta interval. x holds the start on entry.
-template <int MAXD>
-__device__ __forceinline__ bool run_chain(const float* __restrict__ Ap, const float* __restrict__ bp, int F, int dim,
-                                          int mixing, uint32_t k0, uint32_t k1, uint32_t chain, uint32_t stream,
-                                          float* x) {
-  float dir[MAXD];
-#pragma unroll
-  for (int k = 0; k < MAXD; ++k) dir[k] = 0.f;
-  for (int step = 0; step < mixing; ++step) {
-    float ut;
-    step_draws<MAXD>(k0, k1, chain, stream, (uint32_t)step, dim, dir, &ut);
-    float tmax = FLT_MAX, tmin = -FLT_MAX;
-    for (int f = 0; f < F; ++f) {
-      const float* a = Ap + (int64_t)f * dim;
-      float ax = __fmul_rn(a[0], x[0]);
-      float ad = __fmul_rn(a[0], dir[0]);
-#pragma unroll
-      for (int k = 1; k < MAXD; ++k) {
-        if (k < dim) {
-          float ak = a[k];
-          ax = __fmaf_rn(ak, x[k], ax);
-          ad = __fmaf_rn(ak, dir[k], ad);
-        }
-      }
-      float lb = __fsub_rn(bp[f], ax);
-      if (ad < 0.0f)
-        tmin = fmaxf(tmin, __fdiv_rn(lb, ad));
-      else if (ad > 0.0f)
-        tmax = fminf(tmax, __fdiv_rn(lb, ad));
-    }
-    if (isinf(tmax) || isinf(tmin) || tmax < tmin) return false;
-    double th = __dadd_rn(__dmul_rn((double)ut, __dsub_rn(__dmul_rn(0.999999, (double)tmax), (double)tmin)),
-                          (double)tmin);
-    float theta = __double2float_rn(th);
-#pragma unroll
-    for (int k = 0; k < MAXD; ++k)
-      if (k < dim) x[k] = __fmaf_rn(theta, dir[k], x[k]);
-  }
-  return true;
-}
-
 // ---- packed FP32 pairs (sm_100 f32x2): each half is an IEEE round-to-nearest
 // operation, so a packed result is bit for bit the two scalar results.
 __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
@@ -262,7 +220,12 @@ __host__ __device__ __forceinline__ int pair_group_width(int g, int P, int KP) {
 // quotients' residuals and (with the sign taken into theta) the slack and
 // position updates want; negation is exact. A chain whose line search fails keeps stepping without moving (the group's lanes
 // stay convergent) and returns false.
-template <int MAXD, int G, int KP>
+//
+// MAXD: coordinates of a row (8 or 16); NQ: coordinate pairs the dot products
+// run over, at least dim / 2. Coefficients past dim are zero, so they change
+// no dot product, and a count known at compile time spares a test of dim per
+// coordinate.
+template <int MAXD, int NQ, int G, int KP>
 __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, int P, int dim, int mixing,
                                                 uint32_t k0, uint32_t k1, uint32_t chain, uint32_t stream,
                                                 float* xl, int gl, GroupScratch* gs, int bar_id) {
@@ -329,11 +292,11 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
       }
     }
     const int base = t * JB;  // lane of this step's block 0
-    uint64_t dd[MAXD];        // (-dir_k, -dir_k)
+    uint64_t dd[2 * NQ];      // (-dir_k, -dir_k); past dim: any finite number
     float ut;
     if constexpr (G <= 32) {
 #pragma unroll
-      for (int k = 0; k < MAXD; ++k) {
+      for (int k = 0; k < 2 * NQ; ++k) {
         // coordinate k: pair k >> 1 = block k >> 2, half (k >> 1) & 1, cosine or sine k & 1
         const float v = ((k >> 1) & 1) ? ((k & 1) ? c1b : c0b) : ((k & 1) ? c1a : c0a);
         const float dk = __shfl_sync(0xffffffffu, v, base + (k >> 2), G);
@@ -345,8 +308,8 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
       const float* db = gs->dir[batch & 1][t];
       if (t == 0) group_bar(bar_id, G);  // the batch's draws are in scratch
 #pragma unroll
-      for (int k = 0; k < MAXD; ++k) {
-        const float dk = db[k];  // entries past dim are never used
+      for (int k = 0; k < 2 * NQ; ++k) {
+        const float dk = db[k];
         dd[k] = f2_pack(dk, dk);
       }
       ut = db[16];
@@ -362,12 +325,10 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
       const ulonglong2* row = reinterpret_cast<const ulonglong2*>(rows + (size_t)p * RS);
       uint64_t acc = 0ull;
 #pragma unroll
-      for (int q = 0; q < MAXD / 2; ++q) {
-        if (2 * q < dim) {
-          const ulonglong2 v = row[q];  // coordinates 2q and 2q + 1 of both faces
-          acc = q == 0 ? f2_mul(v.x, dd[0]) : f2_fma(v.x, dd[2 * q], acc);
-          if (2 * q + 1 < dim) acc = f2_fma(v.y, dd[2 * q + 1], acc);
-        }
+      for (int q = 0; q < NQ; ++q) {
+        const ulonglong2 v = row[q];  // coordinates 2q and 2q + 1 of both faces
+        acc = q == 0 ? f2_mul(v.x, dd[0]) : f2_fma(v.x, dd[2 * q], acc);
+        acc = f2_fma(v.y, dd[2 * q + 1], acc);
       }
       na2[j] = acc;
       theta_bits(tb, s, acc);
@@ -454,7 +415,7 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
 // lanes per chain; groups past `last` repeat the last chain and store
 // nothing, so every group takes the same number of trips (wide groups meet
 // at named barriers 1 + group index). A failed chain stores `start`.
-template <int MAXD, int G, int KP>
+template <int MAXD, int NQ, int G, int KP>
 __device__ __forceinline__ void sample_chains_pairs(const float* __restrict__ rows, int P, int dim,
                                                     const float* __restrict__ start, int first, int last, int mixing,
                                                     uint32_t k0, uint32_t k1, uint32_t stream,
@@ -462,6 +423,11 @@ __device__ __forceinline__ void sample_chains_pairs(const float* __restrict__ ro
   constexpr int XL = (MAXD + G - 1) / G;
   const int gl = threadIdx.x & (G - 1), gid = threadIdx.x / G, ngroups = blockDim.x / G;
   GroupScratch* gs = G > 32 ? gsa + gid : nullptr;
+  if constexpr (G > 32) {  // directions past dim stay zero (they meet zero coefficients and must be finite)
+    float* d = &gs->dir[0][0][0];
+    for (int i = gl; i < 2 * kDrawSteps * 17; i += G) d[i] = 0.f;
+    group_bar(1 + gid, G);
+  }
   for (int c0 = first; c0 < last; c0 += ngroups) {
     const int chain = c0 + gid;
     const int cc = chain < last ? chain : last - 1;
@@ -471,7 +437,7 @@ __device__ __forceinline__ void sample_chains_pairs(const float* __restrict__ ro
       const int k = gl + G * r;
       xl[r] = k < dim ? start[k] : 0.f;
     }
-    const bool ok = run_chain_pairs<MAXD, G, KP>(rows, P, dim, mixing, k0, k1, (uint32_t)cc, stream, xl, gl, gs,
+    const bool ok = run_chain_pairs<MAXD, NQ, G, KP>(rows, P, dim, mixing, k0, k1, (uint32_t)cc, stream, xl, gl, gs,
                                                  1 + gid);
     if (chain < last) {
 #pragma unroll
@@ -485,30 +451,45 @@ __device__ __forceinline__ void sample_chains_pairs(const float* __restrict__ ro
 
 // The chains of one region with G lanes each (G from pair_group_width, one of
 // 8 .. 256).
-template <int MAXD, int KP>
-__device__ __forceinline__ void sample_region(int G, const float* __restrict__ rows, int P, int dim,
+template <int MAXD, int NQ, int KP>
+__device__ __forceinline__ void sample_region_q(int G, const float* __restrict__ rows, int P, int dim,
                                               const float* __restrict__ start, int first, int last, int mixing,
                                               uint32_t k0, uint32_t k1, uint32_t stream, float* __restrict__ out,
                                               GroupScratch* gsa) {
   switch (G) {
     case 8:
-      sample_chains_pairs<MAXD, 8, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
+      sample_chains_pairs<MAXD, NQ, 8, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
       break;
     case 16:
-      sample_chains_pairs<MAXD, 16, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
+      sample_chains_pairs<MAXD, NQ, 16, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
       break;
     case 32:
-      sample_chains_pairs<MAXD, 32, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
+      sample_chains_pairs<MAXD, NQ, 32, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
       break;
     case 64:
-      sample_chains_pairs<MAXD, 64, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
+      sample_chains_pairs<MAXD, NQ, 64, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
       break;
     case 128:
-      sample_chains_pairs<MAXD, 128, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
+      sample_chains_pairs<MAXD, NQ, 128, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
       break;
     default:
-      sample_chains_pairs<MAXD, 256, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
+      sample_chains_pairs<MAXD, NQ, 256, KP>(rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
       break;
+  }
+}
+
+template <int MAXD, int KP>
+__device__ __forceinline__ void sample_region(int G, const float* __restrict__ rows, int P, int dim,
+                                              const float* __restrict__ start, int first, int last, int mixing,
+                                              uint32_t k0, uint32_t k1, uint32_t stream, float* __restrict__ out,
+                                              GroupScratch* gsa) {
+  if constexpr (MAXD == 16) {
+    if (dim <= 14)
+      sample_region_q<16, 7, KP>(G, rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
+    else
+      sample_region_q<16, 8, KP>(G, rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
+  } else {
+    sample_region_q<8, 4, KP>(G, rows, P, dim, start, first, last, mixing, k0, k1, stream, out, gsa);
   }
 }
 

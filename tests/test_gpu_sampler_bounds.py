@@ -103,3 +103,28 @@ def test_odd_domains_equal_oracle_replay(dim, faces, case):
         A, b, scale = np.delete(A, [0, 2], 0), np.delete(b, [0, 2]), np.delete(scale, [0, 2])
     dom = csd.HPolyhedron((A * scale[:, None]).astype(np.float32), (b * scale).astype(np.float32))
     compare(sc, q0, q1, dom, 800)
+
+
+# lanes per chain 32, 16, 8; one chain to several rounds per block; faces below, at and beyond a lane each, odd
+# counts, and past the staging buffer (48 KB: 1,228 faces at up to 8 dimensions, 682 above)
+@pytest.mark.parametrize("dim", [1, 2, 3, 7, 8, 9, 14, 16])
+@pytest.mark.parametrize("samples,polytopes", [(1, 1), (33, 3), (1000, 5), (9001, 2), (21000, 1)])
+def test_uniform_samples_equal_oracle(dim, samples, polytopes):
+    rng = np.random.default_rng(100 * dim + samples)
+    polys, starts = [], []
+    for i in range(polytopes):
+        n = int(rng.choice([0, 1, 2, 15, 16, 17, 64, 333])) if samples > 33 else [3, 1300, 700][i]
+        a = rng.normal(size=(n, dim))
+        a /= np.linalg.norm(a, axis=1, keepdims=True)
+        c = rng.uniform(-0.5, 0.5, dim)
+        A = np.concatenate([np.kron(np.eye(dim), [[-1.0], [1.0]]), a]).astype(np.float32)
+        b = np.concatenate([np.full(2 * dim, 1.0), a @ c + rng.uniform(0.0, 1.0, n)]).astype(np.float32)
+        if i == 1:  # a start on a face: its slack is too small for the packed quotients
+            b[1] = np.float32(c[0])
+        polys.append(csd.HPolyhedron(A, b))
+        starts.append(c.astype(np.float32))
+    mixing = 3 if samples > 5000 else 12
+    got = csd.UniformSampleInHPolyhedraCuda(polys, np.stack(starts, 1), samples, mixing, seed=dim)
+    for i, (p, x) in enumerate(zip(polys, starts)):
+        ref, _ = O.hit_and_run(p.A(), p.b(), x, samples, mixing, seed=dim, stream=i)
+        np.testing.assert_array_equal(got[i].T, ref)
