@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(1024) batch_step_kernel(BatchArgs a) {
 __global__ void __launch_bounds__(mlp::kThreads) batch_score_kernel(BatchArgs a) {
   extern __shared__ __align__(1024) char smem_raw[];
   char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t bars[2];
+  __shared__ uint64_t bars[mlp::kFwdBars];
   __shared__ uint32_t tmem_base;
   if ((int)blockIdx.y >= a.it->num_act) return;
   const int slot = a.act[blockIdx.y];
@@ -504,15 +504,14 @@ __global__ void __launch_bounds__(mlp::kThreads) batch_score_kernel(BatchArgs a)
   G.dim = S.dim;
   G.net = S.plant;
   G.logits = a.scores + (size_t)slot * a.n_max;
-  const mlp::FwdArgs fa{nullptr, reinterpret_cast<const mlp::bf16*>(a.mlp_wb), a.mlp_params, a.mlp_scale, a.status};
+  const mlp::FwdArgs fa{nullptr, 0, reinterpret_cast<const mlp::bf16*>(a.mlp_wb), a.mlp_params, a.mlp_scale, a.status};
   const int warp = threadIdx.x >> 5;
   if (warp == 0) {
     umma::tmem_alloc(&tmem_base, mlp::kH);
     umma::tmem_relinquish();
   }
   if (threadIdx.x == 0) {
-    umma::bar_init(&bars[0], 1);
-    umma::bar_init(&bars[1], 1);
+    for (int i = 0; i < mlp::kFwdBars; ++i) umma::bar_init(&bars[i], 1);
     umma::bar_fence_init();
   }
   umma::fence_before_sync();

@@ -60,20 +60,29 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
   extern __shared__ __align__(1024) char smem_raw[];
   char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int kA = 128 * kKC * 2, kB = NT * kKC * 2, kStage = kA + kB;
-  __shared__ uint64_t bars[2];
+  __shared__ uint64_t bars[kStages];
   __shared__ uint32_t tmem_base;
   constexpr uint32_t kCols = NT < 32 ? 32 : NT;
   const int grp = blockIdx.z, m0 = blockIdx.x * 128, n0 = blockIdx.y * NT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bf16* A = g.A + grp * g.a_group;
   const bf16* B = g.B + grp * g.b_group;
+  const int nchunks = (g.K + kKC - 1) / kKC;
+  auto load = [&](int c) {
+    if (c < nchunks) {
+      char* sa = smem + (c % kStages) * kStage;
+      load_tile<128, kKC>(A, g.lda, g.M, g.K, m0, c * kKC, sa);
+      load_tile<NT, kKC>(B, g.ldb, g.N, g.K, n0, c * kKC, sa + kA);
+    }
+    umma::copy_commit();  // (an empty group past the end keeps the count)
+  };
+  for (int c = 0; c < kStages - 1; ++c) load(c);
   if (warp == 0) {
     umma::tmem_alloc(&tmem_base, kCols);
     umma::tmem_relinquish();
   }
   if (threadIdx.x == 0) {
-    umma::bar_init(&bars[0], 1);
-    umma::bar_init(&bars[1], 1);
+    for (int i = 0; i < kStages; ++i) umma::bar_init(&bars[i], 1);
     umma::bar_fence_init();
   }
   umma::fence_before_sync();
@@ -81,62 +90,96 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
   umma::fence_after_sync();
   const uint32_t tmem = tmem_base;
   const uint32_t idesc = umma::instr_desc_bf16(128, NT);
-  const int nchunks = (g.K + kKC - 1) / kKC;
   bool ok = true;
-  for (int c = 0; c < nchunks && ok; ++c) {
-    const int st = c & 1;
-    char* sa = smem + st * kStage;
-    char* sb = sa + kA;
-    if (c >= 2) ok = umma::bar_wait(&bars[st], ((c - 2) >> 1) & 1);
+  for (int c = 0; c < nchunks; ++c) {
+    char* sa = smem + (c % kStages) * kStage;
+    umma::copy_wait<kStages - 2>();  // chunk c has arrived
+    umma::fence_smem_async();
     if (!__syncthreads_and(ok)) {
       ok = false;
       break;
     }
-    load_tile(A, g.lda, g.M, g.K, m0, c * kKC, 128, kKC, sa);
-    load_tile(B, g.ldb, g.N, g.K, n0, c * kKC, NT, kKC, sb);
-    umma::fence_smem_async();
-    __syncthreads();
     if (threadIdx.x == 0) {
       umma::fence_after_sync();
       const int steps = min(kKC, g.K - c * kKC + 15) >> 4;
       for (int s = 0; s < steps; ++s)
-        umma::mma_bf16(tmem, umma::tile_desc(umma::smem_u32(sa), s, kKC), umma::tile_desc(umma::smem_u32(sb), s, kKC),
-                       idesc, (c > 0 || s > 0) ? 1u : 0u);
-      umma::commit(&bars[st]);
+        umma::mma_bf16(tmem, umma::tile_desc(umma::smem_u32(sa), s, kKC),
+                       umma::tile_desc(umma::smem_u32(sa + kA), s, kKC), idesc, (c > 0 || s > 0) ? 1u : 0u);
+      umma::commit(&bars[c % kStages]);
     }
+    // chunk c + 3 goes where chunk c - 1 was: once its MMAs are done
+    if (c > 0) ok = umma::bar_wait(&bars[(c - 1) % kStages], ((c - 1) / kStages) & 1);
+    load(c + kStages - 1);
   }
-  if (ok && nchunks > 0) ok = umma::bar_wait(&bars[(nchunks - 1) & 1], ((nchunks - 1) >> 1) & 1);
-  if (nchunks > 1 && ok) ok = umma::bar_wait(&bars[(nchunks - 2) & 1], ((nchunks - 2) >> 1) & 1);
+  umma::copy_wait<0>();
+  // the last commit covers every MMA
+  if (ok && nchunks > 0) ok = umma::bar_wait(&bars[(nchunks - 1) % kStages], ((nchunks - 1) / kStages) & 1);
   if (!__syncthreads_and(ok)) {
     if (threadIdx.x == 0 && g.status) atomicExch(g.status, 1);
   } else {
     umma::fence_after_sync();
     // epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31; warps w and w + 4 split the columns
-    const int row = m0 + 32 * (warp & 3) + lane;
+    const int rw = m0 + 32 * (warp & 3), row = rw + lane;
     constexpr int kSplit = NT >= 32 ? 2 : 1;
-    const int cpw = NT / kSplit;
-    if (warp < 4 * kSplit) {
-      for (int j0 = (warp >> 2) * cpw; j0 < (warp >> 2) * cpw + cpw; j0 += 16) {
+    const int cpw = NT / kSplit, jb = (warp >> 2) * cpw;
+    if (warp < 4 * kSplit && g.epi == kEpiF32) {
+      // through a padded tile (the stages are free), so that a store covers 64 bytes of two rows: a row per lane
+      // touched 32 sectors per store (93 us a launch of 64 nets x 256 x 256)
+      float* tile = reinterpret_cast<float*>(smem) + warp * 32 * 17;
+      float* d = g.D + grp * g.d_group;
+      for (int j0 = jb; j0 < jb + cpw; j0 += 16) {
+        float v[16];
+        umma::tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)j0, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) tile[lane * 17 + i] = v[i];
+        __syncwarp();
+        const int n = n0 + j0 + (lane & 15);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int r = 2 * i + (lane >> 4);
+          if (rw + r < g.M && n < g.N) d[(size_t)(rw + r) * g.ldd + n] = tile[r * 17 + (lane & 15)];
+        }
+        __syncwarp();
+      }
+    } else if (warp < 4 * kSplit) {
+      const bf16* mt = g.mask_t + grp * g.mt_group;
+      bf16 mk[16], mnext[16];
+      auto masks = [&](int j0, bf16* m) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int n = n0 + j0 + i;
+          m[i] = row < g.M && n < g.N ? mt[(size_t)n * g.ldmt + row] : __float2bfloat16_rn(0.f);
+        }
+      };
+      masks(jb, mnext);
+      for (int j0 = jb; j0 < jb + cpw; j0 += 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) mk[i] = mnext[i];
+        if (j0 + 16 < jb + cpw) masks(j0 + 16, mnext);  // one step ahead: their latency is the loop's
         float v[16];
         umma::tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)j0, v);
         if (row < g.M) {
-          if (g.epi == kEpiF32) {
-            float* d = g.D + grp * g.d_group + (size_t)row * g.ldd;
+          uint32_t h[8];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] *= __bfloat162float(mk[i]) > 0.f ? 1.f : 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) h[i] = pack2(v[2 * i], v[2 * i + 1]);
+          const bf16* hv = reinterpret_cast<const bf16*>(h);
+          if (g.out) {
+            bf16* o = g.out + grp * g.o_group + (size_t)row * g.ldo + n0 + j0;
+            if (n0 + j0 + 16 <= g.N && g.ldo % 8 == 0 && g.o_group % 8 == 0) {
+              *reinterpret_cast<uint4*>(o) = make_uint4(h[0], h[1], h[2], h[3]);
+              *reinterpret_cast<uint4*>(o + 8) = make_uint4(h[4], h[5], h[6], h[7]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (n0 + j0 + i < g.N) o[i] = hv[i];
+            }
+          }
+          if (g.out_t) {
 #pragma unroll
             for (int i = 0; i < 16; ++i)
-              if (n0 + j0 + i < g.N) d[n0 + j0 + i] = v[i];
-          } else {
-            const bf16* mt = g.mask_t + grp * g.mt_group;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const int n = n0 + j0 + i;
-              if (n < g.N) {
-                const float keep = __bfloat162float(mt[(size_t)n * g.ldmt + row]) > 0.f ? 1.f : 0.f;
-                const bf16 h = __float2bfloat16_rn(v[i] * keep);
-                if (g.out) g.out[grp * g.o_group + (size_t)row * g.ldo + n] = h;
-                if (g.out_t) g.out_t[grp * g.ot_group + (size_t)n * g.ldot + row] = h;
-              }
-            }
+              if (n0 + j0 + i < g.N) g.out_t[grp * g.ot_group + (size_t)(n0 + j0 + i) * g.ldot + row] = hv[i];
           }
         }
       }
@@ -149,7 +192,8 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
 
 template <int NT>
 size_t gemm_smem() {
-  return 2 * (size_t)(128 * kKC * 2 + NT * kKC * 2) + 1024;
+  const size_t stages = kStages * (size_t)(128 * kKC * 2 + NT * kKC * 2), tile = 8 * 32 * 17 * sizeof(float);
+  return std::max(stages, tile) + 1024;
 }
 
 template <int NT>
@@ -173,7 +217,7 @@ csd_status_t launch_gemm(const GemmArgs& g, int groups, cudaStream_t st) {
 __global__ void __launch_bounds__(kThreads) mlp_forward_kernel(FwdArgs a) {
   extern __shared__ __align__(1024) char smem_raw[];
   char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t bars[2];
+  __shared__ uint64_t bars[kFwdBars];
   __shared__ uint32_t tmem_base;
   const FwdGroup G = a.groups[blockIdx.y];
   const int row0 = blockIdx.x * 128;
@@ -184,8 +228,7 @@ __global__ void __launch_bounds__(kThreads) mlp_forward_kernel(FwdArgs a) {
     umma::tmem_relinquish();
   }
   if (threadIdx.x == 0) {
-    umma::bar_init(&bars[0], 1);
-    umma::bar_init(&bars[1], 1);
+    for (int i = 0; i < kFwdBars; ++i) umma::bar_init(&bars[i], 1);
     umma::bar_fence_init();
   }
   umma::fence_before_sync();
@@ -214,13 +257,13 @@ csd_status_t launch_forward(const FwdArgs& a, int groups, int max_rows, cudaStre
 
 // ------------------------------------------------------- CUDA-core kernels
 // dlogit = (sigmoid(z) - y) / B and the BCE-with-logits loss; block per net.
-__global__ void dlogit_kernel(const float* __restrict__ logits, const uint8_t* __restrict__ y, int B,
+__global__ void dlogit_kernel(const float* __restrict__ logits, const uint8_t* __restrict__ y, int y_net, int B,
                               float* __restrict__ dlogit, float* __restrict__ loss) {
   __shared__ float red[32];
   const int net = blockIdx.x;
   float l = 0.f;
   for (int b = threadIdx.x; b < B; b += blockDim.x) {
-    const float z = logits[(size_t)net * B + b], t = y[(size_t)net * B + b] ? 1.f : 0.f;
+    const float z = logits[(size_t)net * B + b], t = y[(size_t)net * y_net + b] ? 1.f : 0.f;
     const float sg = 1.f / (1.f + expf(-z));
     dlogit[(size_t)net * B + b] = (sg - t) / (float)B;
     l += fmaxf(z, 0.f) - z * t + log1pf(expf(-fabsf(z)));
@@ -323,27 +366,68 @@ __global__ void weights_bf16_kernel(const float* __restrict__ params, int nets, 
   }
 }
 
-// Adam (Kingma & Ba 2015) with bias correction; t is the 1-based step.
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, long long n, float lr, float b1, float b2, float eps, float c1,
-                            float c2) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+// Adam (Kingma & Ba 2015) with bias correction (c1, c2 = 1 - beta^step), and the
+// bf16 copies of the updated weights in the same pass. Block (x, net): x <
+// 128 a 32 x 32 tile of W2 or W3, whose transposed copy goes through shared
+// memory (writing it element by element scattered 2-byte stores over 32 rows:
+// 81 us a step for 64 nets on top of Adam's 56); the rest 1,024 of the other
+// parameters. Bound by its traffic, 28 bytes per parameter.
+constexpr int kAdamTiles = 2 * (kH / 32) * (kH / 32), kAdamRest = kH * kIn + 4 * kH + 1;
+__global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, const float* __restrict__ g,
+                                                   float* __restrict__ m, float* __restrict__ v,
+                                                   bf16* __restrict__ wb, float lr, float b1, float b2, float eps,
+                                                   float c1, float c2) {
+  __shared__ bf16 tile[32][33];
+  const int net = blockIdx.y;
+  const size_t base = (size_t)net * kParams;
+  bf16* w = wb + (size_t)net * kBf;
+  auto update = [&](int e) {
+    const size_t i = base + e;
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    p[i] = pi;
+    return pi;
+  };
+  if ((int)blockIdx.x < kAdamTiles) {
+    constexpr int per = kAdamTiles / 2, side = kH / 32;
+    const int layer = blockIdx.x / per, o0 = (blockIdx.x % per) / side * 32, i0 = blockIdx.x % side * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int off = layer ? oW3 : oW2, q = layer ? qW3 : qW2, qt = layer ? qW3t : qW2t;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int o = o0 + ty + 8 * k, i = i0 + tx;
+      const bf16 h = __float2bfloat16_rn(update(off + o * kH + i));
+      w[q + o * kH + i] = h;
+      tile[ty + 8 * k][tx] = h;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[qt + (i0 + ty + 8 * k) * kH + o0 + tx] = tile[tx][ty + 8 * k];
+    return;
+  }
+  const int r0 = (blockIdx.x - kAdamTiles) * 1024 + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = r0 + 256 * k;  // W1, b1 | b2 | b3, w4, b4
+    if (r >= kAdamRest) break;
+    const int e = r < oW2 ? r : r < oW2 + kH ? oB2 + r - oW2 : oB3 + r - oW2 - kH;
+    const float pi = update(e);
+    if (e < oB1) w[qW1 + e] = __float2bfloat16_rn(pi);
   }
 }
 
-// f32 rows [n][dim] -> bf16 rows [n][16] scaled and zero padded
-__global__ void to_bf16_rows_kernel(const float* __restrict__ x, long long n, int dim, float scale,
-                                    bf16* __restrict__ out) {
+// f32 rows [n][dim] of each group -> its bf16 rows [n][16], scaled and zero padded
+__global__ void to_bf16_rows_kernel(const FwdGroup* __restrict__ groups, long long n, float scale) {
+  const FwdGroup G = groups[blockIdx.y];
+  bf16* out = const_cast<bf16*>(G.xb);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n * kIn; t += (long long)gridDim.x * blockDim.x) {
     const long long r = t / kIn;
     const int k = (int)(t % kIn);
-    out[t] = __float2bfloat16_rn(k < dim ? x[r * dim + k] * scale : 0.f);
+    out[t] = __float2bfloat16_rn(k < G.dim ? G.x[r * G.dim + k] * scale : 0.f);
   }
 }
 
@@ -370,7 +454,7 @@ static csd_status_t ensure_batch(csd_mlp_s* h, int B) {
   if (h->batch == B) return CSD_OK;
   const size_t n = (size_t)h->nets, b = (size_t)B;
   csd_status_t s;
-  if ((s = h->xb.reserve(n * b * kIn * 2)) || (s = h->y.reserve(n * b)) || (s = h->logits.reserve(n * b * 4)) ||
+  if ((s = h->logits.reserve(n * b * 4)) ||
       (s = h->dlogit.reserve(n * b * 4)) || (s = h->loss.reserve(n * 4)) || (s = h->xt.reserve(n * kIn * b * 2)) ||
       (s = h->h1t.reserve(n * kH * b * 2)) || (s = h->h2t.reserve(n * kH * b * 2)) ||
       (s = h->h3t.reserve(n * kH * b * 2)) || (s = h->dz3.reserve(n * b * kH * 2)) ||
@@ -381,14 +465,18 @@ static csd_status_t ensure_batch(csd_mlp_s* h, int B) {
   return CSD_OK;
 }
 
-// forward (training outputs) + backward into h->grads for the batch in h->xb / h->y
-static csd_status_t forward_backward(csd_mlp_s* h, int B, cudaStream_t st) {
+// Groups of the training passes: f32 rows x (net i's at x[i]) converted to bf16
+// rows xb (stride net_rows per net), training outputs of a batch of B rows;
+// uploads them and converts the rows.
+static csd_status_t prepare_rows(csd_mlp_s* h, const float* x, bf16* xb, int net_rows, int B, cudaStream_t st) {
   const int n = h->nets;
   std::vector<FwdGroup> gs(n);
+  size_t off = 0;
   for (int i = 0; i < n; ++i) {
     FwdGroup& G = gs[i];
     G = FwdGroup{};
-    G.xb = h->xb.as<bf16>() + (size_t)i * B * kIn;
+    G.x = x + off;
+    G.xb = xb + (size_t)i * net_rows * kIn;
     G.rows = B;
     G.dim = h->dims[i];
     G.net = i;
@@ -398,14 +486,27 @@ static csd_status_t forward_backward(csd_mlp_s* h, int B, cudaStream_t st) {
     G.h2t = h->h2t.as<bf16>() + (size_t)i * kH * B;
     G.h3t = h->h3t.as<bf16>() + (size_t)i * kH * B;
     G.ld_t = B;
+    off += (size_t)net_rows * h->dims[i];
   }
   csd_status_t s;
   if ((s = h->groups.reserve(gs.size() * sizeof(FwdGroup)))) return s;
   CSD_CUDA_TRY(cudaMemcpyAsync(h->groups.ptr, gs.data(), gs.size() * sizeof(FwdGroup), cudaMemcpyHostToDevice, st));
-  FwdArgs fa{h->groups.as<FwdGroup>(), h->wb.as<bf16>(), h->params.as<float>(), h->in_scale, h->status.as<int>()};
+  CSD_CHECK(n <= 65535, CSD_ERR_CAPACITY, "more than 65535 nets");
+  const int blocks = (int)std::min<long long>(((long long)net_rows * kIn + 255) / 256, 64);
+  to_bf16_rows_kernel<<<dim3(blocks, n), 256, 0, st>>>(h->groups.as<FwdGroup>(), net_rows, h->in_scale);
+  CSD_CUDA_TRY(cudaGetLastError());
+  return CSD_OK;
+}
+
+// forward (training outputs) + backward into h->grads for rows [row0, row0 + B) of the prepared groups; labels
+// y (net i's at y + i y_net), mean losses per net to `loss`
+static csd_status_t forward_backward(csd_mlp_s* h, int B, int row0, const uint8_t* y, int y_net, float* loss,
+                                     cudaStream_t st) {
+  const int n = h->nets;
+  csd_status_t s;
+  FwdArgs fa{h->groups.as<FwdGroup>(), row0, h->wb.as<bf16>(), h->params.as<float>(), h->in_scale, h->status.as<int>()};
   if ((s = launch_forward(fa, n, B, st))) return s;
-  dlogit_kernel<<<n, 256, 0, st>>>(h->logits.as<float>(), h->y.as<uint8_t>(), B, h->dlogit.as<float>(),
-                                   h->loss.as<float>());
+  dlogit_kernel<<<n, 256, 0, st>>>(h->logits.as<float>(), y, y_net, B, h->dlogit.as<float>(), loss);
   out_backward_kernel<<<dim3(kH / 32, n), 256, 0, st>>>(h->h3t.as<bf16>(), h->dlogit.as<float>(),
                                                          h->params.as<float>(), B, h->grads.as<float>(),
                                                          h->dz3.as<bf16>(), h->dz3t.as<bf16>());
@@ -610,7 +711,7 @@ csd_status_t csd_mlp_infer(csd_mlp_t h, int32_t groups, const int32_t* net, cons
   DevBuf dg;
   if ((s = dg.reserve(gs.size() * sizeof(FwdGroup) + 16))) return s;
   CSD_CUDA_TRY(cudaMemcpyAsync(dg.ptr, gs.data(), gs.size() * sizeof(FwdGroup), cudaMemcpyHostToDevice, st));
-  FwdArgs fa{dg.as<FwdGroup>(), h->wb.as<bf16>(), h->params.as<float>(), h->in_scale, h->status.as<int>()};
+  FwdArgs fa{dg.as<FwdGroup>(), 0, h->wb.as<bf16>(), h->params.as<float>(), h->in_scale, h->status.as<int>()};
   if ((s = launch_forward(fa, groups, max_rows, st))) return s;
   if (!dev) CSD_CUDA_TRY(cudaMemcpyAsync(logits, ld, total_r * 4, cudaMemcpyDeviceToHost, st));
   return check_status(h, st);
@@ -623,19 +724,16 @@ csd_status_t csd_mlp_gradients(csd_mlp_t h, const float* x, const uint8_t* y, in
   DeviceScope ds(h->device);
   csd_status_t s;
   if ((s = ensure_batch(h, batch))) return s;
-  size_t off = 0;
   DevBuf dx;
   size_t total = 0;
   for (int i = 0; i < h->nets; ++i) total += (size_t)batch * h->dims[i];
-  if ((s = dx.reserve(total * 4))) return s;
+  if ((s = dx.reserve(total * 4)) || (s = h->xb.reserve((size_t)h->nets * batch * kIn * 2)) ||
+      (s = h->y.reserve((size_t)h->nets * batch)))
+    return s;
   CSD_CUDA_TRY(cudaMemcpy(dx.ptr, x, total * 4, cudaMemcpyHostToDevice));
-  for (int i = 0; i < h->nets; ++i) {
-    to_bf16_rows_kernel<<<256, 256>>>(dx.as<float>() + off, batch, h->dims[i], h->in_scale,
-                                      h->xb.as<bf16>() + (size_t)i * batch * kIn);
-    off += (size_t)batch * h->dims[i];
-  }
   CSD_CUDA_TRY(cudaMemcpy(h->y.ptr, y, (size_t)h->nets * batch, cudaMemcpyHostToDevice));
-  if ((s = forward_backward(h, batch, 0))) return s;
+  if ((s = prepare_rows(h, dx.as<float>(), h->xb.as<bf16>(), batch, batch, 0))) return s;
+  if ((s = forward_backward(h, batch, 0, h->y.as<uint8_t>(), batch, h->loss.as<float>(), 0))) return s;
   if ((s = check_status(h, 0))) return s;
   CSD_CUDA_TRY(cudaMemcpy(grads, h->grads.ptr, (size_t)h->nets * kParams * 4, cudaMemcpyDeviceToHost));
   if (loss) CSD_CUDA_TRY(cudaMemcpy(loss, h->loss.ptr, (size_t)h->nets * 4, cudaMemcpyDeviceToHost));
@@ -650,37 +748,30 @@ csd_status_t csd_mlp_train(csd_mlp_t h, const float* x, const uint8_t* y, int32_
   cudaStream_t st = (cudaStream_t)stream;
   csd_status_t s;
   if ((s = ensure_batch(h, batch))) return s;
-  // the whole dataset as bf16 rows, then per step copy one contiguous batch per net
-  DevBuf xall;
-  if ((s = xall.reserve((size_t)h->nets * n * kIn * 2))) return s;
-  size_t off = 0;
-  for (int i = 0; i < h->nets; ++i) {
-    to_bf16_rows_kernel<<<1024, 256, 0, st>>>(x + off, n, h->dims[i], h->in_scale,
-                                              xall.as<bf16>() + (size_t)i * n * kIn);
-    off += (size_t)n * h->dims[i];
-  }
-  CSD_CUDA_TRY(cudaGetLastError());
-  const long long P = (long long)h->nets * kParams;
-  std::vector<float> lh(h->nets);
+  // the whole dataset as bf16 rows; a step reads its rows in place, and the losses stay on the device until the
+  // end (a copy per net and step, and a synchronisation per step, cost as much as the kernels)
+  DevBuf xall, losses;
+  if ((s = xall.reserve((size_t)h->nets * n * kIn * 2)) ||
+      (s = losses.reserve((size_t)std::max(steps, 1) * h->nets * 4)) ||
+      (s = prepare_rows(h, x, xall.as<bf16>(), n, batch, st)))
+    return s;
   for (int t = 0; t < steps; ++t) {
     const int start = (int)(((long long)t * batch) % n);
-    for (int i = 0; i < h->nets; ++i) {
-      CSD_CUDA_TRY(cudaMemcpyAsync(h->xb.as<bf16>() + (size_t)i * batch * kIn, xall.as<bf16>() + ((size_t)i * n + start) * kIn,
-                                   (size_t)batch * kIn * 2, cudaMemcpyDeviceToDevice, st));
-      CSD_CUDA_TRY(cudaMemcpyAsync(h->y.as<uint8_t>() + (size_t)i * batch, y + (size_t)i * n + start, batch,
-                                   cudaMemcpyDeviceToDevice, st));
-    }
-    if ((s = forward_backward(h, batch, st))) return s;
+    if ((s = forward_backward(h, batch, start, y + start, n, losses.as<float>() + (size_t)t * h->nets, st))) return s;
     h->step += 1;
     const float c1 = 1.f - std::pow(0.9f, (float)h->step), c2 = 1.f - std::pow(0.999f, (float)h->step);
-    adam_kernel<<<2048, 256, 0, st>>>(h->params.as<float>(), h->grads.as<float>(), h->m.as<float>(), h->v.as<float>(),
-                                      P, lr, 0.9f, 0.999f, 1e-8f, c1, c2);
-    if ((s = refresh_bf16(h, st))) return s;
-    if (loss_history) {
-      CSD_CUDA_TRY(cudaMemcpyAsync(lh.data(), h->loss.ptr, (size_t)h->nets * 4, cudaMemcpyDeviceToHost, st));
-      CSD_CUDA_TRY(cudaStreamSynchronize(st));
+    adam_kernel<<<dim3(kAdamTiles + (kAdamRest + 1023) / 1024, h->nets), 256, 0, st>>>(
+        h->params.as<float>(), h->grads.as<float>(), h->m.as<float>(), h->v.as<float>(), h->wb.as<bf16>(), lr, 0.9f,
+        0.999f, 1e-8f, c1, c2);
+    CSD_CUDA_TRY(cudaGetLastError());
+  }
+  if (loss_history && steps > 0) {
+    std::vector<float> lh((size_t)steps * h->nets);
+    CSD_CUDA_TRY(cudaMemcpyAsync(lh.data(), losses.ptr, lh.size() * 4, cudaMemcpyDeviceToHost, st));
+    CSD_CUDA_TRY(cudaStreamSynchronize(st));
+    for (int t = 0; t < steps; ++t) {
       double m = 0;
-      for (float v : lh) m += v;
+      for (int i = 0; i < h->nets; ++i) m += lh[(size_t)t * h->nets + i];
       loss_history[t] = (float)(m / h->nets);
     }
   }

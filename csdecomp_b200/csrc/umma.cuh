@@ -76,6 +76,17 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
                : "memory");
 }
 
+// ---- asynchronous 16-byte copies global -> shared (generic proxy: a reader of the async proxy needs
+// fence_smem_async after the wait); `ok` false fills with zeros and reads nothing
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
 // ---- mbarrier
 __device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
