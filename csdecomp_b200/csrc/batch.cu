@@ -333,13 +333,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) batch_c
     const WarpCtx<M> w = batch_ctx<M>(sp, smem4, static_floats);
     const float* smp = a.fpool + S.smp_off;
     uint8_t* flags = a.bpool + S.flag_off;
-    const int last = std::min(Ns, first + c);
-    for (int i = first + warp; i < last; i += nw) {
-      if (lane < sp.dim) w.qs[lane] = smp[(int64_t)i * sp.dim + lane];
-      __syncwarp();
-      const bool hit = check_warp<M>(sp, w, lane, none);
-      if (lane == 0) flags[i] = hit ? 0 : 1;
-    }
+    const int i0 = first + warp * (c / nw);  // c is a multiple of the block's warps
+    check_range<M>(sp, w, smp, i0, std::min(Ns, i0 + c / nw), lane, none,
+                   [&](int64_t i, bool hit) { flags[i] = hit ? 0 : 1; });
   }
 }
 
@@ -390,9 +386,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) batch_b
     if (!block_plant<M>(a, S.plant, &sp, &cur, smem4, &bar)) return;
     const WarpCtx<M> w = batch_ctx<M>(sp, smem4, static_floats);
     const float* ls = a.fpool + S.seg_off;
-    const int last = std::min(S.K, first + c);
-    for (int i = first + warp; i < last; i += nw)
-      bisect_particle<M>(sp, w, i, S.dim, a.bisection, ls, ls + S.dim, none, a.fpool + S.col_off,
+    const int per = c / nw, i0 = first + warp * per, i1 = std::min(S.K, i0 + per), B = warp_batch<M>(sp);
+    for (int i = i0; i < i1; i += B)
+      bisect_particles<M>(sp, w, i, std::min(B, i1 - i), S.dim, a.bisection, [&](int) { return ls; },
+                          [&](int) { return ls + S.dim; }, none, a.fpool + S.col_off,
                           a.fpool + S.col_off + (int64_t)a.num_particles * S.dim, a.fpool + S.dist_off, lane);
   }
 }
@@ -618,10 +615,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) batch_c
     const int last = min(end_s, first + c);
     for (int p = first + warp; p < last; p += nw) {
       const int i = ord[p];
-      if (lane < sp.dim) w.qs[lane] = smp[(int64_t)i * sp.dim + lane];
-      __syncwarp();
-      const bool hit = check_warp<M>(sp, w, lane, none);
-      if (lane == 0) flags[i] = hit ? 0 : 1;
+      check_range<M>(sp, w, smp, i, i + 1, lane, none, [&](int64_t s, bool hit) { flags[s] = hit ? 0 : 1; });
     }
   }
 }
@@ -782,7 +776,7 @@ struct csd_batch_s {
   int static_floats = 0;
   size_t check_smem = 0;
   int check_grid = 0, bisect_grid = 0;
-  int cfg_max = 128, part_max = 8;  // bisection: one particle per warp per item (every block busy)
+  int cfg_max = 128, part_max = 32;  // largest check and bisection items
   int sample_variant = 0;     // tuned (or set) variant
   int large_variant = 1;      // variant chosen once a slot's faces exceeded the tuned variant's staging
   int run_variant = 0;        // variant of the current iterations

@@ -27,12 +27,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) check_p
   if (!w.ok) return;
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += nw) {
-    if (lane < p.dim) w.qs[lane] = q[i * p.dim + lane];
-    __syncwarp();
-    const bool hit = check_warp<M>(p, w, lane, va);
-    if (lane == 0) out[i] = hit ? 0 : 1;
-  }
+  // runs of a warp's batch, shorter when there are not enough configurations for every warp
+  const int64_t per = (n + nw - 1) / nw;
+  const int64_t B = per < warp_batch<M>(p) ? per : warp_batch<M>(p);
+  for (int64_t i = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * B; i < n; i += nw * B)
+    check_range<M>(p, w, q, i, i + B < n ? i + B : n, lane, va, [&](int64_t k, bool hit) { out[k] = hit ? 0 : 1; });
 }
 
 // ------------------------------------------------------------------ edges
@@ -156,16 +155,23 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) check_e
     const int64_t G = (np + 31) / 32;
     bool collided = false;
     int64_t checked = 0;
-    const float a1 = lane < d ? w.q1[lane] : 0.f, a2 = lane < d ? w.q2[lane] : 0.f;
-    for (int64_t v = 0; v < 32 * G && !collided; ++v) {
-      const int64_t k = (v % 32) * G + v / 32;
-      if (k >= np) continue;
-      const float x = edge_coord(a1, a2, np, mode, k);
+    // batches of visits share their FK; a visit past the edge's points repeats the last point and is not checked
+    const int B = warp_batch<M>(p);
+    for (int64_t v0 = 0; v0 < 32 * G && !collided; v0 += B) {
       __syncwarp();
-      if (lane < d) w.qs[lane] = x;
+      for (int c = lane; c < B * d; c += kWarp) {
+        const int g = c / d, k = c - g * d;
+        const int64_t v = v0 + g, pt = (v % 32) * G + v / 32;
+        w.qs[g * kMaxDim + k] = edge_coord(w.q1[k], w.q2[k], np, mode, pt < np ? pt : np - 1);
+      }
       __syncwarp();
-      ++checked;
-      collided = check_warp<M>(p, w, lane, none);
+      fk_configs<M>(p, w, B, lane);
+      for (int g = 0; g < B && !collided; ++g) {
+        const int64_t v = v0 + g;
+        if ((v % 32) * G + v / 32 >= np) continue;
+        ++checked;
+        collided = check_nth<M>(p, w, g, lane, none);
+      }
     }
     if (lane == 0) {
       out[e] = collided ? 0 : 1;
@@ -285,7 +291,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n)
       if (lane < d) w.qs[lane] = x;
       __syncwarp();
       ++checked;
-      collided = check_warp<M>(p, w, lane, none);
+      fk_configs<M>(p, w, 1, lane);
+      collided = check_nth<M>(p, w, 0, lane, none);
     }
     if (lane == 0) {
       out[e] = collided ? 0 : 1;

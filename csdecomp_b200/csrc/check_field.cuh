@@ -33,74 +33,84 @@
 
 namespace csd {
 
-// Per-warp shared memory (floats): slot transforms as rows [slots][3][4], the
-// configuration and two spare ones [3][kMaxDim], world poses (first the
-// joint-local transforms of fk_rows), link capsules [slots][8].
+// Most configurations whose FK a warp runs at once (fk_rows).
+constexpr int kFkBatch = 8;
+static __host__ __device__ __forceinline__ int fk_batch(const DevPlant& p) { return p.field.fk_batch; }
+
+// Per-warp shared memory (floats): slot transforms as rows
+// [batch][slots][3][4], configurations [batch][kMaxDim], two spare ones
+// [2][kMaxDim], world poses (first the sines and cosines of fk_rows), link
+// capsules [slots][8].
 static __host__ __device__ __forceinline__ int field_scratch_floats(const DevPlant& p) {
-  const int a = (p.pose_words + 3) & ~3, b = 12 * p.num_fk;
+  const int a = (p.pose_words + 3) & ~3, b = (2 * fk_batch(p) * p.num_fk + 3) & ~3;
   return a > b ? a : b;
 }
 static __host__ __device__ __forceinline__ int field_warp_floats(const DevPlant& p) {
-  return p.num_slots * 12 + 3 * kMaxDim + field_scratch_floats(p) + 8 * p.num_slots;
+  return fk_batch(p) * (p.num_slots * 12 + kMaxDim) + 2 * kMaxDim + field_scratch_floats(p) + 8 * p.num_slots;
 }
 
-// FK of the configuration in qs into X[slot] as rows (R[r][0..2], t[r]).
+// FK of the m <= fk_batch configurations in qs [m][kMaxDim] into X
+// [m][slots][3][4], rows (R[r][0..2], t[r]); sc: scratch.
 //
-// Joint-local entries first, one per lane: entry e of joint e / 12 at position
-// 4 c + i (i < 3: row i of column c; i = 3: translation c) is
-// fma(cos, A, fma(sin, B, C)) (kind 0), the constant C (kind 1) or
-// fma(q, B, C) (kind 2). Then lane 4 g + r carries row r of the chain that
-// group g follows: per joint twelve FMAs on its parent's row, which it still
-// holds, in the order of check_core.cuh::fk_warp. fk_step gives each group's
-// joint of a step (255: none) and the parent slot (254: the row in registers,
-// 253: the world); bit 31 asks for a barrier because a parent row comes from
-// another group.
-static __device__ __forceinline__ void fk_rows(const DevPlant& p, const float* qs, float* X, float* loc, int lane) {
-  float sj = 0.f, cj = 1.f;
-  if (lane < p.num_fk) {
-    const FkJoint* J = p.fk + lane;
-    const float qj = qs[__ldg(&J->qidx)];
-    if (__ldg(&J->type) == J_REVOLUTE) {
-      sincosf(qj, &sj, &cj);
-    } else {
-      sj = qj;
-      cj = 0.f;
-    }
-  }
-  const int ne = 12 * p.num_fk;
-  for (int e0 = 0; e0 < ne; e0 += kWarp) {
-    const int e = e0 + lane, j = min(e / 12, p.num_fk - 1);
-    const float s = __shfl_sync(kFull, sj, j), c = __shfl_sync(kFull, cj, j);
-    if (e < ne) {
-      const float4 E = __ldg(p.field.fk_entry + e);
-      loc[e] = E.w == 1.f ? E.z : fmaf(c, E.x, fmaf(s, E.y, E.z));
-    }
+// Sines and cosines first, one joint of one configuration per lane. Then the
+// warp's eight groups of four lanes share out the configurations and, on
+// trees with arms side by side, their branches: group h follows branch
+// h % fk_branches of configuration h / fk_branches, and its lane r < 3 carries
+// row r of the branch: per joint the nine local rotation entries, then twelve
+// FMAs on the parent's row, which it still holds unless the joint branches
+// off, each in the order of check_core.cuh::fk_warp. fk_step: joint (255:
+// none), parent slot << 8 (254: the row in registers, 253: the world), bit 31:
+// a parent row of this step comes from another group. Twelve lanes exchanging
+// one configuration's entries took 0.6 of the 2.1 ms of 2^20 free
+// configurations of the 7-DOF arm, eight configurations at once 0.2.
+static __device__ __forceinline__ void fk_rows(const DevPlant& p, const float* qs, int m, float* X, float* sc,
+                                               int lane) {
+  const FieldTables& f = p.field;
+  float2* sc2 = reinterpret_cast<float2*>(sc);
+  const int nf = p.num_fk, ne = m * nf, nb = f.fk_branches;
+  for (int e = lane; e < ne; e += kWarp) {
+    const int g = e / nf;
+    const FkJoint* J = p.fk + (e - g * nf);
+    const float q = qs[g * kMaxDim + __ldg(&J->qidx)];
+    float s = q, c = 0.f;  // prismatic: the joint value itself
+    if (__ldg(&J->type) == J_REVOLUTE) sincosf(q, &s, &c);
+    sc2[e] = make_float2(s, c);
   }
   __syncwarp();
-  const int g = lane >> 2, r = lane & 3;
-  const float4* L4 = reinterpret_cast<const float4*>(loc);
-  float4* X4 = reinterpret_cast<float4*>(X);
+  const int h = lane >> 2, r = lane & 3, g = h / nb;
+  const bool mine = g < m && r < 3;
+  const uint32_t* step = f.fk_step + (h - g * nb);
+  float4* Xg = reinterpret_cast<float4*>(X + g * p.num_slots * 12) + r;
   float4 row = make_float4(0.f, 0.f, 0.f, 0.f);
-  uint32_t next = __ldg(p.field.fk_step + g);
-  for (int s = 0; s < p.field.num_steps; ++s) {
+  uint32_t next = __ldg(step);
+  for (int s = 0; s < f.fk_steps; ++s) {
     const uint32_t w = next;
-    if (s + 1 < p.field.num_steps) next = __ldg(p.field.fk_step + 8 * (s + 1) + g);
-    if (w >> 31) __syncwarp();
+    if (s + 1 < f.fk_steps) next = __ldg(step + (s + 1) * nb);
+    if (w >> 31) __syncwarp();  // set for the whole step
     const int j = w & 255, par = (w >> 8) & 255;
-    if (j != 255 && r < 3) {
-      const float4 a = L4[3 * j], b = L4[3 * j + 1], c = L4[3 * j + 2];  // columns (R0 R1 R2 | t)
-      if (par == 253) {
-        row = r == 0 ? make_float4(a.x, b.x, c.x, a.w) : r == 1 ? make_float4(a.y, b.y, c.y, b.w)
-                                                                : make_float4(a.z, b.z, c.z, c.w);
-      } else {
-        if (par != 254) row = X4[3 * par + r];
-        row = make_float4(fmaf(row.z, a.z, fmaf(row.y, a.y, row.x * a.x)),
-                          fmaf(row.z, b.z, fmaf(row.y, b.y, row.x * b.x)),
-                          fmaf(row.z, c.z, fmaf(row.y, c.y, row.x * c.x)),
-                          fmaf(row.z, c.w, fmaf(row.y, b.w, fmaf(row.x, a.w, row.w))));
-      }
-      X4[3 * j + r] = row;
+    if (!mine || j == 255) continue;
+    const float4* E = f.fk_entry + 9 * j;
+    const float2 v = sc2[g * nf + j];
+    const bool rev = (w >> 16) & 1u;
+    float L[9], t[3];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      const float4 e = __ldg(E + i);
+      L[i] = rev ? fmaf(v.y, e.x, fmaf(v.x, e.y, e.z)) : e.x;
+      if (i < 3) t[i] = e.w;
+      if (i >= 3 && i < 6 && !rev) t[i - 3] = fmaf(e.w, v.x, t[i - 3]);
     }
+    if (par == 253) {
+      row = r == 0 ? make_float4(L[0], L[3], L[6], t[0]) : r == 1 ? make_float4(L[1], L[4], L[7], t[1])
+                                                                  : make_float4(L[2], L[5], L[8], t[2]);
+    } else {
+      if (par != 254) row = Xg[3 * par];
+      row = make_float4(fmaf(row.z, L[2], fmaf(row.y, L[1], row.x * L[0])),
+                        fmaf(row.z, L[5], fmaf(row.y, L[4], row.x * L[3])),
+                        fmaf(row.z, L[8], fmaf(row.y, L[7], row.x * L[6])),
+                        fmaf(row.z, t[2], fmaf(row.y, t[1], fmaf(row.x, t[0], row.w))));
+    }
+    Xg[3 * j] = row;
   }
   __syncwarp();
 }

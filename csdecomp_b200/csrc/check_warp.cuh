@@ -23,7 +23,7 @@ struct WarpCtx {
   const float4* stat;
   const float4* aabb;
   float* X;
-  float* qs;
+  float* qs;   // [warp_batch][kMaxDim]
   float* q1;
   float* q2;
   float* pose;
@@ -35,11 +35,18 @@ static __host__ __device__ __forceinline__ int mode_warp_floats(const DevPlant& 
   return M == kModeField ? field_warp_floats(p) : warp_floats(p);
 }
 
+// Configurations a warp takes at once: fk_configs runs their FK together where
+// the mode can, and their slot transforms and coordinates are kept apart.
+template <int M>
+static __host__ __device__ __forceinline__ int warp_batch(const DevPlant& p) {
+  return M == kModeField ? fk_batch(p) : 1;
+}
+
 template <int M>
 static __device__ __forceinline__ void warp_buffers(const DevPlant& p, float* wbase, WarpCtx<M>& w) {
   w.X = wbase + (threadIdx.x >> 5) * mode_warp_floats<M>(p);
-  w.qs = w.X + p.num_slots * 12;
-  w.q1 = w.qs + kMaxDim;
+  w.qs = w.X + warp_batch<M>(p) * p.num_slots * 12;
+  w.q1 = w.qs + warp_batch<M>(p) * kMaxDim;
   w.q2 = w.q1 + kMaxDim;
   w.pose = w.q2 + kMaxDim;
 }
@@ -61,16 +68,42 @@ static __device__ __forceinline__ WarpCtx<M> warp_setup(const DevPlant& p, float
   return w;
 }
 
-// Whether the configuration in w.qs collides (warp-uniform).
+// FK of the configurations w.qs[0 .. m), m <= warp_batch.
 template <int M>
-static __device__ __forceinline__ bool check_warp(const DevPlant& p, const WarpCtx<M>& w, int lane,
-                                                  const VoxArgs& va) {
-  if (M == kModeField) {
-    fk_rows(p, w.qs, w.X, w.pose, lane);
-    return check_field(p, w.X, w.pose, lane, va);
-  }
-  fk_warp(p, w.qs, w.X, lane);
+static __device__ __forceinline__ void fk_configs(const DevPlant& p, const WarpCtx<M>& w, int m, int lane) {
+  if (M == kModeField)
+    fk_rows(p, w.qs, m, w.X, w.pose, lane);
+  else
+    fk_warp(p, w.qs, w.X, lane);
+}
+
+// Whether configuration g of the last fk_configs collides (warp-uniform).
+template <int M>
+static __device__ __forceinline__ bool check_nth(const DevPlant& p, const WarpCtx<M>& w, int g, int lane,
+                                                 const VoxArgs& va) {
+  if (M == kModeField) return check_field(p, w.X + g * p.num_slots * 12, w.pose, lane, va);
   return check_config(p, w.stat, w.aabb, w.X, w.pose, lane, va);
+}
+
+// Configurations q[i0 .. i1) by one warp: verdict(i, collides) in order.
+template <int M, typename F>
+static __device__ __forceinline__ void check_range(const DevPlant& p, const WarpCtx<M>& w, const float* __restrict__ q,
+                                                   int64_t i0, int64_t i1, int lane, const VoxArgs& va, F verdict) {
+  const int B = warp_batch<M>(p);
+  for (int64_t i = i0; i < i1; i += B) {
+    const int m = (int)(i1 - i < B ? i1 - i : B);
+    __syncwarp();
+    for (int e = lane; e < m * p.dim; e += kWarp) {
+      const int g = e / p.dim;
+      w.qs[g * kMaxDim + e - g * p.dim] = q[i * p.dim + e];
+    }
+    __syncwarp();
+    fk_configs<M>(p, w, m, lane);
+    for (int g = 0; g < m; ++g) {
+      const bool hit = check_nth<M>(p, w, g, lane, va);
+      if (lane == 0) verdict(i + g, hit);
+    }
+  }
 }
 
 // Blocks per SM the check kernels are compiled for.

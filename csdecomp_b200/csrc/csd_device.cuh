@@ -122,9 +122,10 @@ struct FieldTables {
   const LinkPair* link_pairs;
   int num_link_pairs;
   const uint32_t* pairs;    // moving-moving pairs a | b << 16 by link pair
-  const float4* fk_entry;   // [num_fk][12]: joint-local transform entries (A, B, C, kind), see fk_rows
-  const uint32_t* fk_step;  // [num_steps][8]: joint of each lane group and its parent, see fk_rows
-  int num_steps;
+  const float4* fk_entry;   // [num_fk][9]: P, S, T of rotation entry i; w: t[0..2], v[0..2], unused
+  const uint32_t* fk_step;  // [fk_steps][fk_branches]: joints a configuration's lane groups take side by side (fk_rows)
+  int fk_steps, fk_branches;
+  int fk_batch;             // configurations whose FK a warp runs at once: 8 / fk_branches, fewer with many slots
 };
 
 // Plant description passed to kernels by value (pointers are device memory).

@@ -12,7 +12,7 @@
 //                            segment, every bisection step a fused FK + pair
 //                            check of the midpoint with the link-level broad
 //                            phase, distance to the projection (the EI-ZO
-//                            bisection body, bisect_particle)
+//                            bisection body, bisect_particles)
 //   2. edit_faces_kernel    one warp per region: copies the region, drops the
 //                            candidates outside it, then repeatedly takes the
 //                            nearest live candidate (lower index on ties),
@@ -48,10 +48,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n)
   if (!w.ok) return;
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
-  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < K; i += nw) {
-    const size_t s = (size_t)seg[i] * dim;
-    bisect_particle<M>(p, w, i, dim, steps, starts + s, ends + s, va, cols, proj, dist, lane);
-  }
+  const int B = bisect_batch<M>(p, K, nw);
+  for (int i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * B; i < K; i += nw * B)
+    bisect_particles<M>(p, w, i, min(B, K - i), dim, steps, [&](int k) { return starts + (size_t)seg[k] * dim; },
+                        [&](int k) { return ends + (size_t)seg[k] * dim; }, va, cols, proj, dist, lane);
 }
 
 // Region r: faces [face_off[r], face_off[r+1]) of A/b, candidates

@@ -56,8 +56,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) bisect_
   if (!w.ok) return;
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
-  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < K; i += nw)
-    bisect_particle<M>(p, w, i, dim, steps, ls, le, va, cols, proj, dist, lane);
+  const int B = bisect_batch<M>(p, K, nw);
+  for (int i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * B; i < K; i += nw * B)
+    bisect_particles<M>(p, w, i, min(B, K - i), dim, steps, [&](int) { return ls; }, [&](int) { return le; }, va, cols,
+                        proj, dist, lane);
 }
 
 // One block places up to max_faces faces (greedy, nearest collision first).

@@ -59,58 +59,79 @@ static __device__ __forceinline__ void compact_block(const uint8_t* __restrict__
 }
 
 
-// One warp per particle: lane k holds coordinate k of the collision point,
-// its projection and the bisection bounds; each step is a fused FK + check of
-// the midpoint. Dot products are accumulated in coordinate order with
-// fused multiply-adds (the order the CPU restatement uses).
-template <int M>
-static __device__ __forceinline__ void bisect_particle(const DevPlant& p, const WarpCtx<M>& w, int i, int dim,
-                                                       int steps, const float* __restrict__ ls,
-                                                       const float* __restrict__ le, const VoxArgs& va,
-                                                       float* __restrict__ cols, float* __restrict__ proj,
-                                                       float* __restrict__ dist, int lane) {
-  const float* ci = cols + (size_t)i * dim;
-  // projection onto the segment (every lane evaluates the same serial sums)
-  float seg2 = 0.f, a = 0.f;
-  for (int k = 0; k < dim; ++k) {
-    float dk = __fsub_rn(le[k], ls[k]);
-    seg2 = __fmaf_rn(dk, dk, seg2);
-    a = __fmaf_rn(__fsub_rn(ci[k], ls[k]), dk, a);
-  }
-  const float t = fminf(fmaxf(__fdiv_rn(a, seg2), 0.0f), 1.0f);
-  const float omt = __fsub_rn(1.0f, t);
-  float c = 0.f, pr = 0.f, lo = 0.f, hi = 0.f;
-  if (lane < dim) {
-    c = ci[lane];
-    pr = __fmaf_rn(t, le[lane], __fmul_rn(omt, ls[lane]));
-    lo = pr;
-    hi = c;
+// Particles i0 .. i0 + m of one warp (m <= warp_batch), bisected side by side:
+// a step's midpoints share their FK, then each is checked. Lane k holds
+// coordinate k of a particle's bounds (m pairs of registers). starts(i) and ends(i) give particle i's segment. Dot products
+// are accumulated in coordinate order with fused multiply-adds (the order the
+// CPU restatement uses).
+template <int M, typename S0, typename S1>
+static __device__ __forceinline__ void bisect_particles(const DevPlant& p, const WarpCtx<M>& w, int i0, int m, int dim,
+                                                        int steps, S0 starts, S1 ends, const VoxArgs& va,
+                                                        float* __restrict__ cols, float* __restrict__ proj,
+                                                        float* __restrict__ dist, int lane) {
+  constexpr int MB = M == kModeField ? kFkBatch : 1;
+  float lo[MB], hi[MB];  // hi: the collision point so far
+#pragma unroll
+  for (int g = 0; g < MB; ++g) {
+    lo[g] = hi[g] = 0.f;
+    if (g >= m) break;
+    const float* ci = cols + (size_t)(i0 + g) * dim;
+    const float *ls = starts(i0 + g), *le = ends(i0 + g);
+    // projection onto the segment (every lane evaluates the same serial sums)
+    float seg2 = 0.f, a = 0.f;
+    for (int k = 0; k < dim; ++k) {
+      float dk = __fsub_rn(le[k], ls[k]);
+      seg2 = __fmaf_rn(dk, dk, seg2);
+      a = __fmaf_rn(__fsub_rn(ci[k], ls[k]), dk, a);
+    }
+    const float t = fminf(fmaxf(__fdiv_rn(a, seg2), 0.0f), 1.0f);
+    const float omt = __fsub_rn(1.0f, t);
+    if (lane < dim) {
+      hi[g] = ci[lane];
+      lo[g] = __fmaf_rn(t, le[lane], __fmul_rn(omt, ls[lane]));
+      proj[(size_t)(i0 + g) * dim + lane] = lo[g];
+    }
   }
   for (int s = 0; s < steps; ++s) {
-    const float mid = __fmul_rn(0.5f, __fadd_rn(lo, hi));
     __syncwarp();
-    if (lane < dim) w.qs[lane] = mid;
+#pragma unroll
+    for (int g = 0; g < MB; ++g)
+      if (g < m && lane < dim) w.qs[g * kMaxDim + lane] = __fmul_rn(0.5f, __fadd_rn(lo[g], hi[g]));
     __syncwarp();
-    const bool hit = check_warp<M>(p, w, lane, va);
-    if (hit) {
-      hi = mid;
-      c = mid;
-    } else {
-      lo = mid;
+    fk_configs<M>(p, w, m, lane);
+    uint32_t hits = 0;
+    for (int g = 0; g < m; ++g) hits |= check_nth<M>(p, w, g, lane, va) ? 1u << g : 0u;
+#pragma unroll
+    for (int g = 0; g < MB; ++g) {
+      const float mid = __fmul_rn(0.5f, __fadd_rn(lo[g], hi[g]));
+      if ((hits >> g) & 1u)
+        hi[g] = mid;
+      else
+        lo[g] = mid;
     }
   }
   // distance to the projection, coordinates in order
-  __syncwarp();
-  if (lane < dim) w.qs[lane] = __fsub_rn(c, pr);
-  __syncwarp();
-  float s2 = 0.f;
-  for (int k = 0; k < dim; ++k) s2 = __fmaf_rn(w.qs[k], w.qs[k], s2);
-  if (lane < dim) {
-    cols[(size_t)i * dim + lane] = c;
-    proj[(size_t)i * dim + lane] = pr;
+#pragma unroll
+  for (int g = 0; g < MB; ++g) {
+    if (g >= m) break;
+    const size_t at = (size_t)(i0 + g) * dim + lane;
+    __syncwarp();
+    if (lane < dim) w.qs[lane] = __fsub_rn(hi[g], proj[at]);
+    __syncwarp();
+    float s2 = 0.f;
+    for (int k = 0; k < dim; ++k) s2 = __fmaf_rn(w.qs[k], w.qs[k], s2);
+    if (lane < dim) cols[at] = hi[g];
+    if (lane == 0) dist[i0 + g] = __fsqrt_rn(s2);
   }
-  if (lane == 0) dist[i] = __fsqrt_rn(s2);
   __syncwarp();
+}
+
+// Particles per warp at once for K particles over `warps` warps: one each
+// until every warp has some (the particles of a warp are checked one after
+// the other).
+template <int M>
+static __device__ __forceinline__ int bisect_batch(const DevPlant& p, int K, int warps) {
+  return min(warp_batch<M>(p), max(1, K / warps));
 }
 
 // One block places up to max_faces faces (greedy, nearest collision first).

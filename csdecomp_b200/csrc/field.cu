@@ -1,7 +1,6 @@
 // field.cu -- tables of the field path (check_field.cuh), built once per plant:
 // the grid of cells over the world statics (on the device), the probes of the
-// moving capsules, the link capsules, the moving-moving pairs by link pair and
-// the FK schedule.
+// moving capsules, the link capsules and the moving-moving pairs by link pair.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -228,40 +227,24 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
     }
     lps.push_back(lp);
   }
-  // ---- FK: joint-local entries and the schedule of eight lane groups
-  std::vector<float> entry((size_t)dp.num_fk * 48, 0.f);
+  // ---- FK table
+  std::vector<float> entry((size_t)dp.num_fk * 36, 0.f);
   for (int j = 0; j < dp.num_fk; ++j)
-    for (int c = 0; c < 3; ++c)
-      for (int i = 0; i < 4; ++i) {
-        float* e = &entry[(size_t)(12 * j + 4 * c + i) * 4];
-        const FkJoint& J = fk[j];
-        if (i < 3) {
-          const int k = 3 * c + i;
-          if (J.type == J_REVOLUTE) {
-            e[0] = J.P[k];
-            e[1] = J.S[k];
-            e[2] = J.T[k];
-          } else {
-            e[2] = J.P[k];
-            e[3] = 1.f;
-          }
-        } else {
-          e[2] = J.t[c];
-          if (J.type == J_PRISMATIC)
-            e[1] = J.v[c];  // cos = 0, sin = q
-          else
-            e[3] = 1.f;
-        }
-      }
-  std::vector<uint32_t> steps;
-  {
+    for (int i = 0; i < 9; ++i) {
+      float* e = &entry[(size_t)(9 * j + i) * 4];
+      e[0] = fk[j].P[i];
+      e[1] = fk[j].S[i];
+      e[2] = fk[j].T[i];
+      e[3] = i < 3 ? fk[j].t[i] : i < 6 ? fk[j].v[i - 3] : 0.f;
+    }
+  // FK schedule of `width` lane groups per configuration: the joints whose
+  // parents are done, a joint staying with the group that holds its parent's row
+  auto schedule = [&](int width) {
+    std::vector<uint32_t> steps;
     std::vector<int> step_of(dp.num_fk, -1), group_of(dp.num_fk, -1);
-    int last[8];
-    std::fill(last, last + 8, -1);
+    std::vector<int> last(width, -1);
     for (int done = 0, s = 0; done < dp.num_fk; ++s) {
-      int job[8];
-      std::fill(job, job + 8, -1);
-      // a joint whose parent a group handled last stays with it; others take a free group
+      std::vector<int> job(width, -1);
       for (int pass = 0; pass < 2; ++pass)
         for (int j = 0; j < dp.num_fk; ++j) {
           const int par = fk[j].parent;
@@ -270,7 +253,7 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
           if (pass == 0) {
             if (par >= 0 && last[group_of[par]] == par && job[group_of[par]] < 0) g = group_of[par];
           } else {
-            for (int k = 0; k < 8 && g < 0; ++k)
+            for (int k = 0; k < width && g < 0; ++k)
               if (job[k] < 0) g = k;
           }
           if (g < 0) continue;
@@ -279,21 +262,33 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
           group_of[j] = g;
           ++done;
         }
-      uint32_t w[8], sync = 0;
-      for (int g = 0; g < 8; ++g) {
+      uint32_t sync = 0;
+      std::vector<uint32_t> w(width);
+      for (int g = 0; g < width; ++g) {
         const int j = job[g];
         uint32_t par = 253;
         if (j >= 0 && fk[j].parent >= 0) par = last[g] == fk[j].parent ? 254u : (uint32_t)fk[j].parent;
         if (j >= 0 && par < 253) sync = 1u << 31;
-        w[g] = (j < 0 ? 255u : (uint32_t)j) | par << 8;
+        w[g] = (j < 0 ? 255u : (uint32_t)j) | par << 8 | (j >= 0 && fk[j].type == J_REVOLUTE ? 1u << 16 : 0u);
       }
-      for (int g = 0; g < 8; ++g) {
+      for (int g = 0; g < width; ++g) {
         steps.push_back(w[g] | sync);
         if (job[g] >= 0) last[g] = job[g];
       }
     }
+    return steps;
+  };
+  // more groups per configuration while they nearly halve its steps
+  std::vector<uint32_t> steps = schedule(1);
+  f.fk_branches = 1;
+  for (int width = 2; width <= 4; width *= 2) {
+    std::vector<uint32_t> wider = schedule(width);
+    if (10 * (wider.size() / width) > 6 * (steps.size() / f.fk_branches)) break;
+    steps = wider;
+    f.fk_branches = width;
   }
-  f.num_steps = (int)steps.size() / 8;
+  f.fk_steps = (int)steps.size() / f.fk_branches;
+  f.fk_batch = std::min(kFkBatch / f.fk_branches, dp.num_slots <= 8 ? 8 : dp.num_slots <= 16 ? 4 : 2);
   // ---- grid over the part of the padded statics' box that the robot reaches
   if (S > 0) {
     double lo[3], hi[3], vol = 1;
