@@ -21,8 +21,8 @@
 // configurations of the 7-DOF arm in 200 primitives took 9.9 ms, most of it
 // in the group and static sphere tests and in the capsule-static and self
 // pairs: they visit every static or most link pairs whatever the clearance.
-// Work here is per moving geometry, about one cell read each: 2.1 ms (10^6
-// uniform configurations 5.6 -> 1.5 ms, 40,009 edges 18.3 -> 3.4 ms). Still
+// Work here is per moving geometry, about one cell read each: 1.65 ms (10^6
+// uniform configurations 5.6 -> 1.1 ms, 40,009 edges 18.2 -> 2.9 ms). Still
 // bound by instruction issue and by the latency of dependent loads, not by
 // bandwidth. Cells of at most 2^18 per plant (4 MB): the radius plus half a
 // cell diagonal bounds a list, so finer cells list little less.

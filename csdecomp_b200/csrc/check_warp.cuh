@@ -11,7 +11,7 @@ namespace csd {
 // How a configuration is checked. kModeField (spheres and capsules against
 // the statics' grid, check_field.cuh) wherever the plant has the tables and
 // the broad phase is on: a free configuration of the 7-DOF arm in 200
-// primitives costs 2.0 ns there against 9.5 ns with the link-sphere
+// primitives costs 1.6 ns there against 9.5 ns with the link-sphere
 // broad phase. The other two are the pair sweep of check_core.cuh, for plants
 // with moving boxes, more than 1,024 statics or the broad phase switched off
 // (every pair tested): statics staged in shared memory, or read from global
