@@ -13,7 +13,7 @@ csd_status_t build_voxel_tables(csd_plant_s* p, const int32_t* ids, int nr, std:
                                 int* num_other) {
   const int T = p->dp.num_tiles;
   tab->assign(T, 0u);
-  std::vector<uint32_t> other;
+  std::vector<uint32_t> other, caps((p->dp.num_mcap + kWarp - 1) / kWarp, 0u);
   for (int k = 0; k < nr; ++k) {
     int g = ids[k];
     CSD_CHECK(g >= 0 && g < (int)p->host.moving_of_geom.size(), CSD_ERR_INVALID,
@@ -23,11 +23,14 @@ csd_status_t build_voxel_tables(csd_plant_s* p, const int32_t* ids, int nr, std:
       (*tab)[m / kWarp] |= 1u << (m % kWarp);
     } else if (m >= 0) {
       other.push_back((uint32_t)m);
+      const int q = m - p->dp.num_msph;
+      if (q < p->dp.num_mcap) caps[q / kWarp] |= 1u << (q % kWarp);
     } else {
       other.push_back(0x80000000u | (uint32_t)p->host.static_of_geom[g]);
     }
   }
   tab->insert(tab->end(), other.begin(), other.end());
+  tab->insert(tab->end(), caps.begin(), caps.end());
   *num_other = (int)other.size();
   return CSD_OK;
 }
@@ -128,7 +131,7 @@ csd_status_t csd_check_points(csd_plant_t p, const float* q, int64_t n, const fl
     vt.tile_mask = p->vox_tab.as<uint32_t>();
     vt.other = p->vox_tab.as<uint32_t>() + p->dp.num_tiles;
     vt.num_other = no;
-    if ((s = build_voxel_grid(p, voxel_grid_cell(p, tab, vr), &p->vox_grid_buf, &vt, st))) return s;
+    if ((s = build_voxel_grid(p, voxel_reach(p, tab, vr), n, &p->vox_grid_buf, &vt, st))) return s;
   }
   if (flags == CSD_PTR_DEVICE) {
     s = launch_check_points(p, q, n, vt, out, st);

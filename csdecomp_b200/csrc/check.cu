@@ -17,10 +17,11 @@
 
 namespace csd {
 
-template <int M>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) check_points_kernel(DevPlant p, const float* __restrict__ q,
-                                                                          int64_t n, VoxArgs va,
-                                                                          uint8_t* __restrict__ out) {
+// VOX: with voxels (their test costs registers that a check without them would spill).
+template <int M, bool VOX>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n)
+    check_points_kernel(DevPlant p, const float* __restrict__ q, int64_t n, VoxArgs vox, uint8_t* __restrict__ out) {
+  const VoxArgs va = VOX ? vox : VoxArgs{};
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
   const WarpCtx<M> w = warp_setup<M>(p, smem4, &bar);
@@ -434,7 +435,7 @@ csd_status_t launch_check_points(const csd_plant_s* p, const float* q, int64_t n
   if (n <= 0) return CSD_OK;
   const VoxArgs va = vox_args(vt);
   return with_mode(plant_mode(p), [&](auto m) -> csd_status_t {
-    auto kernel = check_points_kernel<decltype(m)::value>;
+    auto kernel = va.nv > 0 ? check_points_kernel<decltype(m)::value, true> : check_points_kernel<decltype(m)::value, false>;
     const size_t smem = smem_bytes(p, kWarpsPerBlock);
     int grid = 0;
     if (csd_status_t s = grid_for(kernel, smem, n, &grid, kWarpsPerBlock)) return s;

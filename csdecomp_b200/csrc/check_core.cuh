@@ -41,18 +41,21 @@ struct VoxArgs {
   const int* gstart;    // [buckets + 1] first voxel of each bucket
   int gmask;            // buckets - 1 (a power of two minus one)
   float ginv_h;         // 1 / cell edge
+  float grins;          // a cell lists the voxels within this of it (0: those inside it)
 };
 
 static inline VoxArgs vox_args(const VoxelTables& vt) {
-  return VoxArgs{vt.vox, vt.nv, vt.vr, vt.tile_mask, vt.other, vt.num_other, vt.gvox, vt.gstart, vt.gmask, vt.ginv_h};
+  return VoxArgs{vt.vox, vt.nv, vt.vr, vt.tile_mask, vt.other, vt.num_other, vt.gvox, vt.gstart, vt.gmask, vt.ginv_h, vt.grins};
 }
 
 // ---- voxel hash grid: cell (floor(x/h), floor(y/h), floor(z/h)) computed as
 // floor(x * inv_h), which is monotone in x, so a voxel within R of a point
-// lies in a cell between the cells of the point -/+ R on every axis. Buckets
-// by the spatial hash of Teschner et al. (2003), "Optimized Spatial Hashing
-// for Collision Detection of Deformable Objects" (primes 73856093, 19349663,
-// 83492791); cells sharing a bucket only add candidates.
+// lies in a cell between the cells of the point -/+ R on every axis. The
+// columns of cells along z are hashed as in Teschner et al. (2003), "Optimized
+// Spatial Hashing for Collision Detection of Deformable Objects" (primes
+// 73856093, 19349663), and the cells of a column take consecutive buckets
+// (modulo their number): a query box reads one run of voxels per column
+// instead of one per cell. Cells sharing a bucket only add candidates.
 static __host__ __device__ __forceinline__ int vox_cell(float x, float inv_h) {
 #ifdef __CUDA_ARCH__
   return __float2int_rd(__fmul_rn(x, inv_h));
@@ -62,7 +65,7 @@ static __host__ __device__ __forceinline__ int vox_cell(float x, float inv_h) {
 #endif
 }
 static __host__ __device__ __forceinline__ uint32_t vox_bucket(int ix, int iy, int iz, int mask) {
-  return ((uint32_t)ix * 73856093u ^ (uint32_t)iy * 19349663u ^ (uint32_t)iz * 83492791u) & (uint32_t)mask;
+  return (((uint32_t)ix * 73856093u ^ (uint32_t)iy * 19349663u) + (uint32_t)iz) & (uint32_t)mask;
 }
 constexpr int kVoxGridMaxCells = 512;   // larger query boxes test every voxel
 constexpr int kVoxGridMinVoxels = 64;   // fewer voxels are tested without a grid
@@ -714,8 +717,9 @@ static __device__ bool sweep_generic(const DevPlant& p, const float4* stat, cons
   return false;
 }
 
-// Voxels near one geometry through the hash grid: every voxel in the cells
-// covering the geometry's bounding sphere (bc, br) grown by the voxel radius
+// Voxels near one geometry through the hash grid: every voxel listed in the
+// cells that the geometry's bounding sphere (bc, br) grown by the voxel radius,
+// less the distance within which cells list voxels, touches
 // (x 1.001 + 1e-4 m, above any FP32 rounding of the pair tests) is tested
 // with the same pair test as the full sweep, so the verdict is the full
 // sweep's. SPH: the geometry is the sphere G (tested as in the tile sweep).
@@ -725,8 +729,8 @@ static __device__ bool grid_geom_hit(const VoxArgs& va, int tg, const float* G, 
   int lo[3], hi[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    lo[i] = vox_cell(__fsub_rn(bc[i], R), va.ginv_h);
-    hi[i] = vox_cell(__fadd_rn(bc[i], R), va.ginv_h);
+    lo[i] = vox_cell(__fsub_rn(bc[i], fmaxf(R - va.grins, 0.f)), va.ginv_h);
+    hi[i] = vox_cell(__fadd_rn(bc[i], fmaxf(R - va.grins, 0.f)), va.ginv_h);
   }
   const long long cells = (long long)(hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1);
   const bool finite = isfinite(bc[0]) && isfinite(bc[1]) && isfinite(bc[2]) && isfinite(R);
@@ -737,17 +741,21 @@ static __device__ bool grid_geom_hit(const VoxArgs& va, int tg, const float* G, 
     }
     return false;
   }
-  for (int ix = lo[0]; ix <= hi[0]; ++ix)
-    for (int iy = lo[1]; iy <= hi[1]; ++iy)
-      for (int iz = lo[2]; iz <= hi[2]; ++iz) {
-        const uint32_t b = vox_bucket(ix, iy, iz, va.gmask);
-        const int k1 = __ldg(va.gstart + b + 1);
+  for (int i = 0; i <= hi[0] - lo[0]; ++i)
+    for (int j = 0; j <= hi[1] - lo[1]; ++j) {
+      int b = (int)vox_bucket(lo[0] + i, lo[1] + j, lo[2], va.gmask);
+      for (int left = min(hi[2] - lo[2], va.gmask) + 1; left > 0;) {  // buckets of the column, in two runs where it wraps
+        const int n = min(left, va.gmask + 1 - b);
+        const int k1 = __ldg(va.gstart + b + n);
         for (int k = __ldg(va.gstart + b); k < k1; ++k) {
           const float4 v = __ldg(va.gvox + k);
           float S[4] = {v.x, v.y, v.z, va.vr};
           if (SPH ? sph_sph_hit(G, S) : pair_hit(G_SPHERE, S, tg, G)) return true;
         }
+        left -= n;
+        b = 0;
       }
+    }
   return false;
 }
 

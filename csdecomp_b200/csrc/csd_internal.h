@@ -100,13 +100,15 @@ struct VoxelTables {
   int nv = 0;
   float vr = 0.f;
   const uint32_t* tile_mask = nullptr;  // [num_tiles] lanes of each sphere tile checked against voxels
-  const uint32_t* other = nullptr;      // geometry refs (bit31 = static) checked lane-over-voxels
+  const uint32_t* other = nullptr;      // geometry refs (bit31 = static) checked lane-over-voxels; with a grid,
+                                        // then the bits of the moving capsules among them
   int num_other = 0;
   // hash grid over the voxels (voxgrid.cu); gstart == nullptr: no grid
   const float4* gvox = nullptr;
   const int* gstart = nullptr;
   int gmask = 0;
   float ginv_h = 0.f;
+  float grins = 0.f;
 };
 
 csd_status_t build_voxel_tables(csd_plant_s* p, const int32_t* robot_ids, int nr, std::vector<uint32_t>* tab,
@@ -122,14 +124,18 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
 // Synchronises st, then reads and clears the plant's status word (capi.cu):
 // CSD_ERR_CUDA when a block's bounded staging wait gave up since the last read.
 csd_status_t plant_status(const csd_plant_s* p, cudaStream_t st);
-// Cell edge of the voxel grid for these tables (tab from build_voxel_tables):
-// twice the median radius of the robot spheres checked against voxels plus
-// the voxel radius.
-float voxel_grid_cell(const csd_plant_s* p, const std::vector<uint32_t>& tab, float vr);
+// Median and largest radius of the robot spheres checked against voxels (tab
+// from build_voxel_tables), each plus the voxel radius.
+struct VoxelReach {
+  float med, max;
+};
+VoxelReach voxel_reach(const csd_plant_s* p, const std::vector<uint32_t>& tab, float vr);
 // Builds the hash grid of the device voxels vt->vox (vt->nv of them) into buf
 // on stream st and fills vt's grid fields, when the plant's grid switch is on
-// and there are at least kVoxGridMinVoxels voxels; otherwise leaves them null.
-csd_status_t build_voxel_grid(const csd_plant_s* p, float cell, DevBuf* buf, VoxelTables* vt, cudaStream_t st);
+// and there are enough voxels; leaves vt->gstart null otherwise. checks: about
+// how many configurations will be tested against it.
+csd_status_t build_voxel_grid(const csd_plant_s* p, VoxelReach reach, int64_t checks, DevBuf* buf, VoxelTables* vt,
+                              cudaStream_t st);
 
 // kernels (check.cu)
 csd_status_t launch_check_points(const csd_plant_s* p, const float* q, int64_t n, const VoxelTables& vt,

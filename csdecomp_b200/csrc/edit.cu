@@ -37,11 +37,12 @@ namespace csd {
 constexpr int kEditFaceThreads = 256;
 constexpr int kEditMaxVoxels = 10000;  // MAX_NUM_VOXELS, cuda_edge_inflation_zero_order.h:13
 
-template <int M>
+template <int M, bool VOX>  // VOX: with voxels
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n)
     edit_bisect_kernel(DevPlant p, int K, int dim, int steps, const float* __restrict__ starts,
-                       const float* __restrict__ ends, const uint32_t* __restrict__ seg, VoxArgs va,
+                       const float* __restrict__ ends, const uint32_t* __restrict__ seg, VoxArgs vox,
                        float* __restrict__ cols, float* __restrict__ proj, float* __restrict__ dist) {
+  const VoxArgs va = VOX ? vox : VoxArgs{};
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
   const WarpCtx<M> w = warp_setup<M>(p, smem4, &bar);
@@ -220,7 +221,8 @@ csd_status_t csd_edit_regions(csd_plant_t plant, const float* collisions, const 
     vtab_dev.tile_mask = vt;
     vtab_dev.other = vt + plant->dp.num_tiles;
     vtab_dev.num_other = num_other;
-    if ((s = build_voxel_grid(plant, voxel_grid_cell(plant, vtab, voxel_radius), &grid_buf, &vtab_dev, st)))
+    if ((s = build_voxel_grid(plant, voxel_reach(plant, vtab, voxel_radius), n * (options->bisection_steps + 1), &grid_buf,
+                              &vtab_dev, st)))
       return s;
   }
   const VoxArgs va = vox_args(vtab_dev);
@@ -228,7 +230,8 @@ csd_status_t csd_edit_regions(csd_plant_t plant, const float* collisions, const 
   // 1. bisection, one warp per collision
   const int K = (int)n, steps = (int)options->bisection_steps;
   s = with_mode(plant_mode(plant), [&](auto md) -> csd_status_t {
-    auto kernel = edit_bisect_kernel<decltype(md)::value>;
+    constexpr int M = decltype(md)::value;
+    auto kernel = va.nv > 0 ? edit_bisect_kernel<M, true> : edit_bisect_kernel<M, false>;
     const size_t smem = smem_bytes(plant, kWarpsPerBlock);
     int grid = 0;
     if (csd_status_t e = grid_for(kernel, smem, K, &grid, kWarpsPerBlock)) return e;

@@ -43,13 +43,11 @@ __global__ void compact_kernel(const uint8_t* __restrict__ flags, const float* _
   compact_block(flags, samples, N, M, max_keep, dim, cols, cnt);
 }
 
-template <int M>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) bisect_kernel(DevPlant p, int K, int dim, int steps,
-                                                                       const float* __restrict__ ls,
-                                                                       const float* __restrict__ le, VoxArgs va,
-                                                                       float* __restrict__ cols,
-                                                                       float* __restrict__ proj,
-                                                                       float* __restrict__ dist) {
+template <int M, bool VOX>  // VOX: with voxels
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n)
+    bisect_kernel(DevPlant p, int K, int dim, int steps, const float* __restrict__ ls, const float* __restrict__ le,
+                  VoxArgs vox, float* __restrict__ cols, float* __restrict__ proj, float* __restrict__ dist) {
+  const VoxArgs va = VOX ? vox : VoxArgs{};
   extern __shared__ float4 smem4[];
   __shared__ uint64_t bar;
   const WarpCtx<M> w = warp_setup<M>(p, smem4, &bar);
@@ -114,7 +112,7 @@ static csd_status_t launch_bisect(const csd_plant_s* p, int K, int dim, int step
                                   const VoxArgs& va, float* cols, float* proj, float* dist, cudaStream_t st) {
   if (K <= 0) return CSD_OK;
   return with_mode(plant_mode(p), [&](auto m) -> csd_status_t {
-    auto kernel = bisect_kernel<decltype(m)::value>;
+    auto kernel = va.nv > 0 ? bisect_kernel<decltype(m)::value, true> : bisect_kernel<decltype(m)::value, false>;
     const size_t smem = smem_bytes(p, kWarpsPerBlock);
     int grid = 0;
     if (csd_status_t s = grid_for(kernel, smem, K, &grid, kWarpsPerBlock)) return s;
@@ -243,7 +241,8 @@ csd_status_t csd_inflator_inflate(csd_inflator_t h, const float* ls, const float
     vt.tile_mask = h->vtab.as<uint32_t>();
     vt.other = h->vtab.as<uint32_t>() + p->dp.num_tiles;
     vt.num_other = h->num_other;
-    if ((s = build_voxel_grid(p, voxel_grid_cell(p, h->vtab_host, vr), &h->vgrid, &vt, st))) return s;
+    if ((s = build_voxel_grid(p, voxel_reach(p, h->vtab_host, vr), (int64_t)o.num_particles * o.bisection_steps, &h->vgrid,
+                              &vt, st))) return s;
   }
   const VoxArgs va = vox_args(vt);
   EizoCounters* cnt = h->cnt.as<EizoCounters>();
