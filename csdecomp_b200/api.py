@@ -555,7 +555,10 @@ def EditRegionsCuda(collisions, line_segment_idxs, line_start_points, line_end_p
     if v.shape[0] > MAX_NUM_VOXELS:
         raise RuntimeError("Voxel buffer size insufficient")
     n = col.shape[1]
-    seg = np.ascontiguousarray(np.asarray(list(line_segment_idxs), np.int64).reshape(-1))
+    if not (isinstance(line_segment_idxs, np.ndarray) and line_segment_idxs.ndim == 1
+            and line_segment_idxs.dtype.kind in "iu" and np.can_cast(line_segment_idxs.dtype, np.int64)):
+        line_segment_idxs = list(line_segment_idxs)
+    seg = np.ascontiguousarray(np.asarray(line_segment_idxs, np.int64).reshape(-1))
     if seg.size != n:
         raise ValueError("one line segment index per collision is required")
     if n and (seg.min() < 0 or seg.max() >= m):

@@ -1062,6 +1062,8 @@ csd_status_t csd_batch_create(const csd_plant_t* plants, int32_t num_plants, int
             "too many slots times samples per iteration");
   h->mode = field ? kModeField : max_static <= kStaticSmemLimit ? kModeStaged : kModeGlobal;
   h->static_floats = h->mode == kModeStaged ? max_static / 4 : 0;
+  if (h->mode == kModeStaged)
+    for (csd_plant_t pl : h->plants) pl->may_stage = true;
   h->check_smem = (size_t)(field ? max_field_wf : max_wf) * sizeof(float) * kWarpsPerBlock +
                   (size_t)h->static_floats * sizeof(float);
   int g1 = 0, g2 = 0, g3 = 0;

@@ -39,6 +39,10 @@ csd_status_t build_voxel_tables(csd_plant_s* p, const int32_t* ids, int nr, std:
 // nonzero when a block's bounded wait for the static-table staging gave up,
 // in which case that block returned without checking its configurations.
 csd_status_t plant_status(const csd_plant_s* p, cudaStream_t st) {
+  if (p->dp.cull && p->dp.has_field && !p->may_stage) {
+    CSD_CUDA_TRY(cudaStreamSynchronize(st));
+    return CSD_OK;
+  }
   int v = 0;
   CSD_CUDA_TRY(cudaMemcpyAsync(&v, p->dp.status, sizeof(int), cudaMemcpyDeviceToHost, st));
   CSD_CUDA_TRY(cudaStreamSynchronize(st));
@@ -139,6 +143,16 @@ csd_status_t csd_check_points(csd_plant_t p, const float* q, int64_t n, const fl
     if (nv > 0 && nr > 0) return plant_status(p, st);  // synchronises: voxel tables are reused per call
     return CSD_OK;
   }
+  const size_t qb = ((size_t)n * d * sizeof(float) + 255) & ~size_t(255);
+  char* map = nullptr;
+  if (n > 0 && n <= kMappedConfigs && !mapped_memory(p, qb + (size_t)n, &map)) {
+    uint8_t* o = reinterpret_cast<uint8_t*>(map + qb);
+    std::memcpy(map, q, (size_t)n * d * sizeof(float));
+    if ((s = launch_check_points(p, reinterpret_cast<const float*>(map), n, vt, o, st))) return s;
+    if ((s = plant_status(p, st))) return s;
+    std::memcpy(out, o, (size_t)n);
+    return CSD_OK;
+  }
   if ((s = p->in_buf.reserve((size_t)n * d * sizeof(float) + 16))) return s;
   if ((s = p->out_buf.reserve((size_t)n + 16))) return s;
   if (n * d) CSD_CUDA_TRY(cudaMemcpyAsync(p->in_buf.ptr, q, (size_t)n * d * sizeof(float), cudaMemcpyHostToDevice, st));
@@ -159,6 +173,7 @@ csd_status_t csd_plant_wait_selftest(csd_plant_t p, int32_t polls, int32_t* repo
   CSD_CHECK(p && reported && polls >= 1, CSD_ERR_INVALID, "bad arguments");
   DeviceGuard g(p->device);
   *reported = 0;
+  p->may_stage = true;
   staging_wait_selftest_kernel<<<1, 128, 0, 0>>>(p->dp.status, (long long)polls);
   CSD_CUDA_TRY(cudaGetLastError());
   const csd_status_t s = plant_status(p, 0);
@@ -396,15 +411,15 @@ csd_status_t csd_uniform_sample_hpolyhedra(const float* A, const float* b, const
          bs = (size_t)P * dim * sizeof(float), bout = (size_t)P * S * dim * sizeof(float);
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
   size_t total = al(bA) + al(bb) + al(bo) + al(bs) + al(bout) + 256;
-  char* dev = nullptr;
-  CSD_CUDA_TRY(cudaMalloc((void**)&dev, total));
-  char* pA = dev;
+  CallScratch dev(st);
+  csd_status_t s = dev.reserve(total);
+  if (s) return s;
+  char* pA = dev.as<char>();
   char* pb = pA + al(bA);
   char* po = pb + al(bb);
   char* ps = po + al(bo);
   char* pout = ps + al(bs);
   int* pnf = reinterpret_cast<int*>(pout + al(bout));
-  csd_status_t s = CSD_OK;
   auto h2d = [&](void* dst, const void* src, size_t n) {
     if (!s && n && cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st) != cudaSuccess) {
       set_error("cudaMemcpyAsync failed");
@@ -426,7 +441,7 @@ csd_status_t csd_uniform_sample_hpolyhedra(const float* A, const float* b, const
     set_error("copy back failed");
     s = CSD_ERR_CUDA;
   }
-  cudaFree(dev);
+  if (!s) dev.settled();
   if (num_failed) *num_failed = nf;
   return s;
 }

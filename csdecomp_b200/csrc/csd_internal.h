@@ -46,6 +46,40 @@ struct DevBuf {
   T* as() const { return reinterpret_cast<T*>(ptr); }
 };
 
+// Device memory of one call without a handle of its own, on the current
+// device: taken from blocks kept by earlier calls, or allocated. The destructor
+// waits for the stream's work unless settled() says that the caller has, and
+// keeps the block for later calls while at most kScratchKept bytes of a device
+// are kept; the last csd_plant_destroy frees them. Calls on several threads and
+// streams each hold their own block. (cudaMalloc and cudaFree cost a call
+// about 10 us.)
+class CallScratch {
+ public:
+  explicit CallScratch(cudaStream_t st) : st_(st) {}
+  CallScratch(const CallScratch&) = delete;
+  CallScratch& operator=(const CallScratch&) = delete;
+  ~CallScratch();
+  csd_status_t reserve(size_t n);
+  void settled() { settled_ = true; }
+  template <typename T>
+  T* as() const { return reinterpret_cast<T*>(ptr_); }
+
+ private:
+  cudaStream_t st_;
+  void* ptr_ = nullptr;
+  size_t bytes_ = 0;
+  int dev_ = 0;
+  bool settled_ = false;
+};
+constexpr size_t kScratchKept = size_t(32) << 20;
+
+// Host-pointer point checks of at most this many configurations run on mapped
+// host memory: no copy is launched, the kernel reads the configurations and
+// writes the verdicts over the bus. Against copies (whole call): 33
+// configurations 39.4 -> 27.5 us, 1,024 37.1 -> 30.1, 10,000 67.5 -> 48.8. The
+// line keeps a plant's pinned memory at 2 MB; the copies' share shrinks beyond.
+constexpr int64_t kMappedConfigs = 16384;
+
 struct HostPlant {  // host copies kept for host-side checks and voxel tables
   int dim = 0;
   int num_links = 0;
@@ -86,9 +120,13 @@ struct csd_plant_s {
   void* blob = nullptr;  // device tables
   void* field_blob = nullptr;  // device tables of the field path (field.cu)
   bool cull_eligible = false;  // <= 32 slots and <= 1024 statics
+  bool may_stage = false;      // the pair sweep may have run (its bounded staging wait can set dp.status)
   bool vox_grid = true;        // voxel checks through the hash grid (csd_plant_set_voxel_grid)
   // scratch for host-pointer calls and per-call voxel tables
   csd::DevBuf in_buf, in_buf2, out_buf, out_buf2, vox_buf, vox_tab, vox_grid_buf, counter;
+  void* mapped = nullptr;  // host memory the device reads and writes (small host-pointer calls)
+  size_t mapped_bytes = 0;
+  csd_plant_s();
   ~csd_plant_s();
 };
 
@@ -123,7 +161,10 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
                          const std::vector<double>& static_box, const std::vector<double>& reach_box);
 // Synchronises st, then reads and clears the plant's status word (capi.cu):
 // CSD_ERR_CUDA when a block's bounded staging wait gave up since the last read.
+// A plant whose checks have all run on the field path has nothing to read.
 csd_status_t plant_status(const csd_plant_s* p, cudaStream_t st);
+// The plant's mapped host memory, grown to `bytes` (the device must be done with it).
+csd_status_t mapped_memory(csd_plant_s* p, size_t bytes, char** ptr);
 // Median and largest radius of the robot spheres checked against voxels (tab
 // from build_voxel_tables), each plus the voxel radius.
 struct VoxelReach {

@@ -175,7 +175,9 @@ csd_status_t csd_edit_regions(csd_plant_t plant, const float* collisions, const 
   const size_t sz_vox = al((size_t)std::max(nv, 1) * 12), sz_vt = al((vtab.size() + 1) * 4);
   const size_t total = 2 * sz_cols + sz_dist + sz_seg + 2 * sz_ends + sz_A + sz_b + 2 * sz_off + sz_Ao + sz_bo +
                        sz_nf + sz_vox + sz_vt;
-  DevBuf buf, grid_buf;
+  const cudaStream_t st = 0;
+  CallScratch buf(st);
+  DevBuf grid_buf;
   if ((s = buf.reserve(total))) return s;
   char* base = buf.as<char>();
   size_t off = 0;
@@ -199,7 +201,6 @@ csd_status_t csd_edit_regions(csd_plant_t plant, const float* collisions, const 
   int* nfd = (int*)take(sz_nf);
   float* vox = (float*)take(sz_vox);
   uint32_t* vt = (uint32_t*)take(sz_vt);
-  const cudaStream_t st = 0;
   CSD_CUDA_TRY(cudaMemcpyAsync(cols, grouped.data(), (size_t)n * d * 4, cudaMemcpyHostToDevice, st));
   CSD_CUDA_TRY(cudaMemcpyAsync(seg, gseg.data(), (size_t)n * 4, cudaMemcpyHostToDevice, st));
   CSD_CUDA_TRY(cudaMemcpyAsync(ls, line_starts, (size_t)m * d * 4, cudaMemcpyHostToDevice, st));
@@ -212,7 +213,8 @@ csd_status_t csd_edit_regions(csd_plant_t plant, const float* collisions, const 
   CSD_CUDA_TRY(cudaMemcpyAsync(coffd, coff.data(), (size_t)(m + 1) * 4, cudaMemcpyHostToDevice, st));
   if (nv) CSD_CUDA_TRY(cudaMemcpyAsync(vox, voxels, (size_t)nv * 12, cudaMemcpyHostToDevice, st));
   if (!vtab.empty()) CSD_CUDA_TRY(cudaMemcpyAsync(vt, vtab.data(), vtab.size() * 4, cudaMemcpyHostToDevice, st));
-  CSD_CUDA_TRY(cudaMemsetAsync(plant->dp.status, 0, 4, st));
+  const bool staged = plant_mode(plant) != kModeField;  // only the pair sweep's staging wait can give up
+  if (staged) CSD_CUDA_TRY(cudaMemsetAsync(plant->dp.status, 0, 4, st));
   VoxelTables vtab_dev;
   if (nv > 0) {
     vtab_dev.vox = vox;
@@ -221,8 +223,8 @@ csd_status_t csd_edit_regions(csd_plant_t plant, const float* collisions, const 
     vtab_dev.tile_mask = vt;
     vtab_dev.other = vt + plant->dp.num_tiles;
     vtab_dev.num_other = num_other;
-    if ((s = build_voxel_grid(plant, voxel_reach(plant, vtab, voxel_radius), n * (options->bisection_steps + 1), &grid_buf,
-                              &vtab_dev, st)))
+    if ((s = build_voxel_grid(plant, voxel_reach(plant, vtab, voxel_radius), n * (options->bisection_steps + 1),
+                              &grid_buf, &vtab_dev, st)))
       return s;
   }
   const VoxArgs va = vox_args(vtab_dev);
@@ -247,12 +249,13 @@ csd_status_t csd_edit_regions(csd_plant_t plant, const float* collisions, const 
   CSD_CUDA_TRY(cudaGetLastError());
   int kstat = 0;
   CSD_CUDA_TRY(cudaMemcpyAsync(num_faces, nfd, (size_t)m * 4, cudaMemcpyDeviceToHost, st));
-  CSD_CUDA_TRY(cudaMemcpyAsync(&kstat, plant->dp.status, 4, cudaMemcpyDeviceToHost, st));
+  if (staged) CSD_CUDA_TRY(cudaMemcpyAsync(&kstat, plant->dp.status, 4, cudaMemcpyDeviceToHost, st));
   CSD_CUDA_TRY(cudaMemcpyAsync(A_out, Ao, cap * d * 4, cudaMemcpyDeviceToHost, st));
   CSD_CUDA_TRY(cudaMemcpyAsync(b_out, bo, cap * 4, cudaMemcpyDeviceToHost, st));
   CSD_CUDA_TRY(cudaMemcpyAsync(projections, proj, (size_t)n * d * 4, cudaMemcpyDeviceToHost, st));
   CSD_CUDA_TRY(cudaMemcpyAsync(optimized_collisions, cols, (size_t)n * d * 4, cudaMemcpyDeviceToHost, st));
   CSD_CUDA_TRY(cudaStreamSynchronize(st));
+  buf.settled();
   CSD_CHECK(kstat == 0, CSD_ERR_CUDA, "static geometry staging timed out in the bisection kernel");
   return CSD_OK;
 }

@@ -36,6 +36,90 @@ DevBuf::~DevBuf() {
   if (ptr) cudaFree(ptr);
 }
 
+namespace {
+struct ScratchBlock {
+  void* ptr;
+  size_t bytes;
+  int dev;
+};
+std::mutex scratch_mu;
+std::vector<ScratchBlock> scratch_blocks;  // kept by CallScratch
+int scratch_plants = 0;                    // plants that exist
+
+void scratch_trim() {  // with scratch_mu held
+  int cur = 0;
+  cudaGetDevice(&cur);
+  for (const ScratchBlock& b : scratch_blocks) {
+    cudaSetDevice(b.dev);
+    cudaFree(b.ptr);
+  }
+  cudaSetDevice(cur);
+  scratch_blocks.clear();
+}
+
+void scratch_plant(int n) {  // one plant more or less
+  std::lock_guard<std::mutex> lock(scratch_mu);
+  scratch_plants += n;
+  if (n < 0 && scratch_plants == 0) scratch_trim();
+}
+}  // namespace
+
+csd_status_t CallScratch::reserve(size_t n) {
+  cudaGetDevice(&dev_);
+  n = (std::max<size_t>(n, 1) + 65535) & ~size_t(65535);
+  {
+    std::lock_guard<std::mutex> lock(scratch_mu);
+    int best = -1;
+    for (int i = 0; i < (int)scratch_blocks.size(); ++i) {
+      const ScratchBlock& b = scratch_blocks[i];
+      if (b.dev == dev_ && b.bytes >= n && (best < 0 || b.bytes < scratch_blocks[best].bytes)) best = i;
+    }
+    if (best >= 0) {
+      ptr_ = scratch_blocks[best].ptr;
+      bytes_ = scratch_blocks[best].bytes;
+      scratch_blocks.erase(scratch_blocks.begin() + best);
+      return CSD_OK;
+    }
+  }
+  CSD_CUDA_TRY(cudaMalloc(&ptr_, n));
+  bytes_ = n;
+  return CSD_OK;
+}
+
+CallScratch::~CallScratch() {
+  if (!ptr_) return;
+  if (!settled_ && cudaStreamSynchronize(st_) != cudaSuccess) {
+    cudaFree(ptr_);
+    return;
+  }
+  std::lock_guard<std::mutex> lock(scratch_mu);
+  size_t kept = bytes_;
+  for (const ScratchBlock& b : scratch_blocks)
+    if (b.dev == dev_) kept += b.bytes;
+  if (kept <= kScratchKept)
+    scratch_blocks.push_back({ptr_, bytes_, dev_});
+  else
+    cudaFree(ptr_);
+}
+
+csd_status_t mapped_memory(csd_plant_s* p, size_t bytes, char** ptr) {
+  if (p->mapped_bytes < bytes) {
+    if (p->mapped) cudaFreeHost(p->mapped);
+    p->mapped = nullptr;
+    p->mapped_bytes = 0;
+    size_t n = 65536;
+    while (n < bytes) n <<= 1;
+    if (cudaHostAlloc(&p->mapped, n, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();  // the caller copies instead
+      p->mapped = nullptr;
+      return CSD_ERR_CUDA;
+    }
+    p->mapped_bytes = n;
+  }
+  *ptr = reinterpret_cast<char*>(p->mapped);
+  return CSD_OK;
+}
+
 int device_sm_count() {
   static std::mutex mu;
   static int cache[64] = {0};
@@ -230,9 +314,13 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 }  // namespace
 }  // namespace csd
 
+csd_plant_s::csd_plant_s() { csd::scratch_plant(1); }
+
 csd_plant_s::~csd_plant_s() {
   if (blob) cudaFree(blob);
   if (field_blob) cudaFree(field_blob);
+  if (mapped) cudaFreeHost(mapped);
+  csd::scratch_plant(-1);
 }
 
 using namespace csd;
@@ -875,6 +963,7 @@ csd_status_t csd_plant_destroy(csd_plant_t p) {
 csd_status_t csd_plant_set_culling(csd_plant_t p, int32_t enable) {
   CSD_CHECK(p, CSD_ERR_INVALID, "null plant");
   p->dp.cull = (enable && p->cull_eligible) ? 1 : 0;
+  p->may_stage = true;
   return CSD_OK;
 }
 
