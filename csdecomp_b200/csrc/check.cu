@@ -6,11 +6,12 @@
 // re-multiplies two 4x4 transforms per pair (cuda_collision_checker.cu:16-64),
 // and poolPairCollisionFreeResultsKernel ANDs the N*P byte flags (:66-85).
 //
-// Here one warp checks one configuration end to end (check_core.cuh): FK,
-// placement and the pair sweep stay in registers and shared memory, the
-// static geometry is staged into shared memory once per block, and a warp
-// vote stops the sweep at the first colliding pair. Only the configurations
-// and the verdict bytes touch HBM.
+// Here one warp checks up to eight configurations end to end: FK of all of
+// them side by side, then each one's placement and tests, in registers and
+// shared memory; a warp vote stops at the first colliding pair. The statics
+// are found through a grid (check_field.cuh) or, in the pair sweep
+// (check_core.cuh), staged into shared memory once per block. Only the
+// configurations and the verdict bytes touch HBM.
 #include <algorithm>
 
 #include "check_warp.cuh"

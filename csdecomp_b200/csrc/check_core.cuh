@@ -67,7 +67,9 @@ static __host__ __device__ __forceinline__ int vox_cell(float x, float inv_h) {
 static __host__ __device__ __forceinline__ uint32_t vox_bucket(int ix, int iy, int iz, int mask) {
   return (((uint32_t)ix * 73856093u ^ (uint32_t)iy * 19349663u) + (uint32_t)iz) & (uint32_t)mask;
 }
-constexpr int kVoxGridMaxCells = 512;   // larger query boxes test every voxel
+// Larger query boxes test every voxel. A box is read column by column (256 of 16 cells at the limit); 512 sent
+// spheres of 0.4 m to the full sweep once cells are half as wide (voxgrid.cu).
+constexpr int kVoxGridMaxCells = 4096;
 constexpr int kVoxGridMinVoxels = 64;   // fewer voxels are tested without a grid
 
 // Per-warp shared memory (floats): slot transforms [slots][12], the warp's

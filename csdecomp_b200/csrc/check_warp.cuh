@@ -1,6 +1,6 @@
-// check_warp.cuh -- the warp-per-configuration kernels' view of a plant: which
-// check runs (mode), the per-warp shared memory, FK and check of one
-// configuration, launch sizes.
+// check_warp.cuh -- the checking warps' view of a plant: which check runs
+// (mode), the per-warp shared memory, FK and check of a few configurations,
+// launch sizes.
 #pragma once
 #include <type_traits>
 
@@ -137,8 +137,8 @@ static inline csd_status_t with_mode(int mode, F f) {
 // Blocks of a launch. The blocks per SM of a kernel, device and size are asked
 // for once per thread (a few entries, replaced in turn): the queries of
 // attributes and occupancy, with the read of the staging status, cost a small
-// call 12 us of 52. Shared-memory limits only ever rise, so
-// one seen raised stays raised.
+// call 12 us of 52. Shared-memory limits only ever rise, so one seen raised
+// stays raised.
 template <typename K>
 static csd_status_t grid_for(K kernel, size_t smem, int64_t work_warps, int* grid, int wpb) {
   struct Seen {

@@ -9,10 +9,10 @@
 //
 // Here the editing is two launches after one upload:
 //   1. edit_bisect_kernel   one warp per collision: projection onto its own
-//                            segment, every bisection step a fused FK + pair
-//                            check of the midpoint with the link-level broad
-//                            phase, distance to the projection (the EI-ZO
-//                            bisection body, bisect_particles)
+//                            segment, every bisection step a fused FK +
+//                            collision check of the midpoint, distance to the
+//                            projection (the EI-ZO bisection body,
+//                            bisect_particles)
 //   2. edit_faces_kernel    one block per region: copies the region, drops the
 //                            candidates outside it, then repeatedly takes the
 //                            nearest live candidate (lower index on ties),

@@ -10,7 +10,7 @@
 // Here an iteration is five launches and one 16-byte device-to-host read:
 //   1. sample_region_kernel         M_k chains in the current region (face-pair
 //                                    rows, slacks carried from step to step)
-//   2. check_points_kernel          fused FK + pair sweep, one verdict byte each
+//   2. check_points_kernel          fused FK + collision check, one verdict byte each
 //   3. compact_kernel               one block: ordered prefix scan of the
 //                                    colliding samples (the reference's atomicAdd
 //                                    slot order is scheduling dependent,
@@ -19,7 +19,8 @@
 //   -- host reads the counts, applies the admissibility test --
 //   4. bisect_kernel                projection onto the segment and all
 //                                    bisection steps, each step a fused FK +
-//                                    check of the 32 midpoints a warp owns
+//                                    check of the midpoints a warp owns (one,
+//                                    or a few where there are more than warps)
 //   5. faces_kernel                 one block: greedy argmin (first index on
 //                                    ties, as thrust::min_element), face
 //                                    placement with the segment relaxation

@@ -455,10 +455,10 @@ uint32_t csd_num_samples_unadaptive(float epsilon, float delta, float tau);
 /* Diagnostics (no counterpart in the reference): FP32 FMA throughput of the
  * current device, the denominator of the collision kernels' roofline. */
 csd_status_t csd_fp32_fma_probe(int64_t iters, double* flops, double* seconds);
-/* Link-level broad phase of the collision checks (no counterpart in the
- * reference, which tests every pair): per configuration, each moving link's
- * bounding sphere is placed in the world and pairs whose link or static
- * bounding spheres are apart by more than 1e-4 m are skipped. Verdicts are
+/* Broad phase of the collision checks (no counterpart in the reference, which
+ * tests every pair): pairs apart by more than 1e-4 m are skipped, found through
+ * a grid over the statics and capsules around the links or, for plants with
+ * moving boxes, through bounding spheres of links and statics. Verdicts are
  * unchanged. On by default for plants with at most 32 moving links and 1024
  * static geometries; enable = 0 evaluates every pair (the full sweep that
  * csd_plant_flops counts). Takes effect for later calls and for batches
@@ -468,8 +468,8 @@ csd_status_t csd_plant_set_culling(csd_plant_t plant, int32_t enable);
  * and csd_inflator_inflate with voxels, csd_edit_regions; the reference tests
  * every robot geometry against every voxel, cuda_collision_checker.cu:374-435):
  * per call the voxels are bucketed on the device by a spatial hash of their
- * cells, and each robot geometry tests only the voxels in the cells its
- * bounding sphere touches. Used for 64 voxels or more; verdicts are
+ * cells, and each robot geometry tests only the voxels listed in the cells
+ * that spheres around it touch. Used for 64 voxels or more; verdicts are
  * unchanged. On by default; enable = 0 tests every voxel. */
 csd_status_t csd_plant_set_voxel_grid(csd_plant_t plant, int32_t enable);
 
