@@ -799,11 +799,12 @@ struct csd_batch_s {
   csd::DevBuf scores, order, status;
   std::vector<long long> job_configs;  // configurations checked per inflation of the last call
   std::vector<int> act_host;
-  // captured iterations by samplers launched (kSampleStaged | kSampleRegs)
+  // captured iterations by samplers launched (kSampleStaged | kSampleRegs), each with what its capture fixed:
+  // the kernels' arguments by value and the sampler variant
   struct IterationGraph {
     cudaGraphExec_t exec = nullptr;
-    int slots = -1, cfg = -1, variant = -1;
-    const void* mlp = nullptr;
+    csd::BatchArgs args;
+    int variant = -1;
     int kernels = 0;            // kernel nodes
   } graphs[4];
   cudaStream_t reg_stream = nullptr;  // the register sampler's branch of an iteration
@@ -973,11 +974,11 @@ int launch_iteration(csd_batch_s* h, int num_slots, const BatchArgs& a, cudaStre
   return sample_kernels + (a.mlp_wb ? 3 + 2 * a.rounds : 2) + 3;
 }
 
-// The captured iteration with these samplers (captured again when a shape changed).
+// The captured iteration with these samplers (captured again when any argument
+// of its kernels changed: the surrogate's stop rule, rounds and pointers are among them).
 csd_status_t build_graph(csd_batch_s* h, int num_slots, const BatchArgs& a, int samplers) {
   csd_batch_s::IterationGraph& G = h->graphs[samplers];
-  if (G.exec && G.slots == num_slots && G.cfg == a.cfg_max && G.variant == h->run_variant && G.mlp == a.mlp_wb)
-    return CSD_OK;
+  if (G.exec && G.variant == h->run_variant && std::memcmp(&G.args, &a, sizeof a) == 0) return CSD_OK;
   if (G.exec) {
     cudaGraphExecDestroy(G.exec);
     G.exec = nullptr;
@@ -998,10 +999,8 @@ csd_status_t build_graph(csd_batch_s* h, int num_slots, const BatchArgs& a, int 
     set_error(std::string("graph instantiation failed: ") + cudaGetErrorString(e));
     return CSD_ERR_CUDA;
   }
-  G.slots = num_slots;
-  G.cfg = a.cfg_max;
+  std::memcpy(&G.args, &a, sizeof a);
   G.variant = h->run_variant;
-  G.mlp = a.mlp_wb;
   return CSD_OK;
 }
 
@@ -1218,7 +1217,8 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
   *h->host_iter = zero;
   CSD_CUDA_TRY(cudaMemcpyAsync(h->iter.ptr, h->host_iter, sizeof(BatchIter), cudaMemcpyHostToDevice, st));
   CSD_CUDA_TRY(cudaMemcpyAsync(h->act.ptr, h->act_host.data(), (size_t)ns * 4, cudaMemcpyHostToDevice, st));
-  BatchArgs a{};
+  BatchArgs a;
+  std::memset(&a, 0, sizeof a);  // padding too: build_graph compares the bytes
   a.slots = h->slots_dev.as<SlotState>();
   a.plants = h->plants_dev.as<DevPlant>();
   a.num_slots = ns;
@@ -1565,7 +1565,6 @@ csd_status_t csd_batch_set_surrogate_rounds(csd_batch_t h, int32_t rounds, int32
             "rounds must be in [1, 8] and the first round at least 32 samples");
   h->rounds = rounds;
   h->round_base = first_round;
-  for (csd_batch_s::IterationGraph& g : h->graphs) g.slots = -1;
   return CSD_OK;
 }
 
