@@ -267,13 +267,18 @@ static __device__ int place_faces(int K, int dim, int max_faces, int nf, int cap
         const int md = pair_maxd(dim), h = nf & 1;
         float* r = rows + (size_t)(nf >> 1) * pair_stride(dim);
         const float slack = __fsub_rn(bb, v0);
+        const float big = __any_sync(0xffffffffu, lane < dim && !(fabsf(a) <= kMaxCoeff)) ? 1.f : 0.f;
         if (lane < md) {
           r[2 * lane + h] = lane < dim ? a : 0.f;
           if (!h) r[2 * lane + 1] = lane < dim ? a : 0.f;
         }
         if (lane == 0) {
           r[2 * md + h] = slack;
-          if (!h) r[2 * md + 1] = slack;
+          r[2 * md + 2 + h] = big;
+          if (!h) {
+            r[2 * md + 1] = slack;
+            r[2 * md + 3] = big;
+          }
         }
       }
     }

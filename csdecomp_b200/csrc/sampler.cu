@@ -44,13 +44,17 @@ __global__ void __launch_bounds__(256, NQ <= 4 ? 4 : 2)
   const float* Ap = A + (int64_t)f0 * dim;
   const float* bp = b + f0;
   const bool staged = (size_t)P * RS * sizeof(float) <= kUniformStageBytes;
+  bool packed = staged;  // the packed quotients serve: staged, and no coefficient beyond kMaxCoeff
   if (staged) {
+    bool big = false;
     for (int i = threadIdx.x; i < 2 * P * MAXD; i += blockDim.x) {
       const int p = i / (2 * MAXD), k = (i >> 1) % MAXD, f = min(2 * p + (i & 1), F - 1);  // an odd count repeats its last face
-      sm[p * RS + 2 * k + (i & 1)] = k < dim ? Ap[(int64_t)f * dim + k] : 0.f;
+      const float v = k < dim ? Ap[(int64_t)f * dim + k] : 0.f;
+      sm[p * RS + 2 * k + (i & 1)] = v;
+      big = big || !(fabsf(v) <= kMaxCoeff);
     }
     for (int i = threadIdx.x; i < 2 * P; i += blockDim.x) sm[(i >> 1) * RS + 2 * MAXD + (i & 1)] = bp[min(i, F - 1)];
-    __syncthreads();
+    packed = !__syncthreads_or(big);
   }
   const int gl = threadIdx.x & (G - 1), ngroups = blockDim.x / G;
   const int npairs = (dim + 1) >> 1, JB = (npairs >> 1) + 1;
@@ -105,7 +109,7 @@ __global__ void __launch_bounds__(256, NQ <= 4 ? 4 : 2)
         s = f2_sub(*reinterpret_cast<const uint64_t*>(sm + p * RS + 2 * MAXD), ax);
       };
       float tmax = FLT_MAX, tmin = -FLT_MAX;
-      for (int pass = staged ? 0 : 1;; ++pass) {
+      for (int pass = packed ? 0 : 1;; ++pass) {
         if (pass == 0) {
           ThetaBits tb = theta_bits_start();
           for (int p = gl; p < P; p += G) {

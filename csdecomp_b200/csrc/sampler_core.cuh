@@ -50,14 +50,19 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
 //
 // Face-pair rows: row p holds faces 2p and 2p + 1 interleaved, coordinate k of
 // face 2p + h at float 2k + h (k < MAXD, zero past dim), the two start slacks
-// at 2 MAXD and 2 MAXD + 1, then two unused floats: 2 MAXD + 4 floats, a
-// multiple of 16 bytes. A face that does not exist yet (the partner of the
+// at 2 MAXD and 2 MAXD + 1, then a mark per face (1: a coefficient is beyond
+// kMaxCoeff, else 0): 2 MAXD + 4 floats, a multiple of 16 bytes. A face that does not exist yet (the partner of the
 // last face of an odd count) holds a copy of that face: it bounds theta
 // exactly as the face does, so it changes no bound. One 16-byte load brings two
 // coordinates of both faces, and one packed FMA (fma.rn.f32x2, each half an
 // IEEE round-to-nearest FMA) advances both faces' dot products.
 __host__ __device__ constexpr int pair_maxd(int dim) { return dim <= 8 ? 8 : 16; }
 __host__ __device__ constexpr int pair_stride(int dim) { return 2 * pair_maxd(dim) + 4; }
+
+// Coefficients up to here leave a . dir finite (a direction's coordinates stay
+// below 8); a face with one beyond, or a NaN, is marked for one division per
+// face, because the packed quotient of an infinite a . dir is NaN, not 0.
+constexpr float kMaxCoeff = 1.2676506002282294e30f;  // 2^100
 
 // Writes face f (coordinates a[0..dim), offset b) of a region whose chains
 // start at x0. An even f also fills its partner half with a copy of itself.
@@ -67,11 +72,17 @@ __device__ __forceinline__ void put_face(float* __restrict__ rows, int dim, int 
   float* r = rows + (size_t)(f >> 1) * pair_stride(dim);
   float ax = __fmul_rn(a[0], x0[0]);
   for (int k = 1; k < dim; ++k) ax = __fmaf_rn(a[k], x0[k], ax);
-  for (int k = 0; k < md; ++k) r[2 * k + h] = k < dim ? a[k] : 0.f;
+  bool big = false;
+  for (int k = 0; k < md; ++k) {
+    r[2 * k + h] = k < dim ? a[k] : 0.f;
+    big = big || (k < dim && !(fabsf(a[k]) <= kMaxCoeff));
+  }
   r[2 * md + h] = __fsub_rn(b, ax);
+  r[2 * md + 2 + h] = big ? 1.f : 0.f;
   if (!h) {  // until face f + 1 is written, its half repeats face f (a face seen twice bounds nothing new)
     for (int k = 0; k < md; ++k) r[2 * k + 1] = r[2 * k];
     r[2 * md + 1] = r[2 * md];
+    r[2 * md + 3] = r[2 * md + 2];
   }
 }
 
@@ -151,8 +162,10 @@ __device__ __forceinline__ void theta_bits(ThetaBits& t, uint64_t s, uint64_t na
 // such a lane takes theta_bound over its faces), and both bounds of the group
 // within [kMinTheta, kMaxTheta), so that the binding a . dir lies in
 // [2^-59, 2^126) and its quotient is exact (otherwise the group takes
-// theta_bound). A face whose a . dir is too small or too large for the packed
-// steps has a quotient outside that range, so it cannot bind unseen.
+// theta_bound). A face whose finite a . dir is too small or too large for the
+// packed steps has a quotient outside that range, so it cannot bind unseen; a
+// lane holding a marked face (kMaxCoeff) takes theta_bound whatever its slacks:
+// its least slack is compared with kNoSlack, which every slack is below.
 //
 // The slow path over n face pairs copied to local memory, in a loop that is
 // not unrolled: the branch is next to never taken, and with the quotients of
@@ -171,6 +184,7 @@ __device__ __forceinline__ void theta_bounds_slow(const uint64_t* s, const uint6
   }
 }
 constexpr float kMinSlack = 9.313225746154785e-10f;   // 2^-30
+constexpr int kNoSlack = 0x7fffffff;
 constexpr float kMinTheta = 7.888609052210118e-31f;   // 2^-100
 constexpr float kMaxTheta = 536870912.f;              // 2^29
 
@@ -240,10 +254,14 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
   // as that pair's owner's (so the group's lanes never diverge in the face loop) and a face seen
   // twice changes no theta bound
   uint64_t s2[KP], na2[KP];  // na2: -(a . dir)
+  int min_slack = __float_as_int(kMinSlack);
 #pragma unroll
   for (int j = 0; j < KP; ++j) {
     const int p = min(gl + G * j, P - 1);
-    s2[j] = P > 0 ? *reinterpret_cast<const uint64_t*>(rows + (size_t)p * RS + 2 * MAXD) : 0ull;
+    ulonglong2 sm = make_ulonglong2(0ull, 0ull);  // slacks, marks
+    if (P > 0) sm = *reinterpret_cast<const ulonglong2*>(rows + (size_t)p * RS + 2 * MAXD);
+    s2[j] = sm.x;
+    if (sm.y) min_slack = kNoSlack;
     na2[j] = 0ull;  // with th = -0 the first update leaves every slack as it is
   }
   float th = -0.0f;
@@ -335,7 +353,7 @@ __device__ __forceinline__ bool run_chain_pairs(const float* __restrict__ rows, 
     }
     float tmax, tmin;
     for (int pass = 0;; ++pass) {
-      if (pass || tb.slack < __float_as_int(kMinSlack)) {  // this lane's faces one division each
+      if (pass || tb.slack < min_slack) {  // this lane's faces one division each
         tmax = FLT_MAX;
         tmin = -FLT_MAX;
         uint64_t ls[KP], ln[KP];
@@ -540,6 +558,7 @@ __device__ __forceinline__ void sample_chains_regs(const float* __restrict__ row
   const int npairs = (dim + 1) >> 1, JB = (npairs >> 1) + 1;
   // this lane's pairs; past the last pair: copies of it (they bound what it bounds)
   uint64_t a[KR][2 * NQ], s0[KR];
+  int min_slack = __float_as_int(kMinSlack);
   const int row0 = reg_row(wig, gid, W);
 #pragma unroll
   for (int j = 0; j < KR; ++j) {
@@ -550,7 +569,9 @@ __device__ __forceinline__ void sample_chains_regs(const float* __restrict__ row
       a[j][2 * q] = v.x;
       a[j][2 * q + 1] = v.y;
     }
-    s0[j] = *reinterpret_cast<const uint64_t*>(r + 32);
+    const ulonglong2 sm = *reinterpret_cast<const ulonglong2*>(r + 32);  // slacks, marks
+    s0[j] = sm.x;
+    if (sm.y) min_slack = kNoSlack;
   }
   // coordinates past dim have zero coefficients; their direction must only be finite
   for (int i = gl; i < 2 * C * S * 32; i += GL) (&sc.dir[0][0][0][0])[i] = 0.f;
@@ -630,7 +651,7 @@ __device__ __forceinline__ void sample_chains_regs(const float* __restrict__ row
       // a slack too small for the packed quotients: theta_max = 0 sends the group to the second pass
 #pragma unroll
       for (int c = 0; c < C; ++c) {
-        tb[c].hi = tb[c].slack < __float_as_int(kMinSlack) ? 0u : tb[c].hi;
+        tb[c].hi = tb[c].slack < min_slack ? 0u : tb[c].hi;
         tb[c].hi = __reduce_min_sync(0xffffffffu, tb[c].hi);
         tb[c].lo = __reduce_min_sync(0xffffffffu, tb[c].lo);
       }
