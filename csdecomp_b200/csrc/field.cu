@@ -17,6 +17,11 @@ constexpr int kFieldMaxStatics = 1024;   // as the broad phase (cull_eligible)
 constexpr double kFieldMinEdge = 0.02;   // finer cells list the same statics
 constexpr double kProbeGrowth = 1.2;     // a probe's radius over its capsule's, at most (more probes below it)
 constexpr int kMaxProbes = 12;           // probes of one capsule
+// Largest coordinates (metres from the world's origin) of a grid's box and of a
+// static's extents: up to there the FP32 rounding of a probe's place in its cell
+// (4 ulp of 128 m on each axis) and of a distance to a static (2 ulp of 256 m)
+// stay below kFieldMargin together.
+constexpr double kFieldGridLimit = 64, kFieldStaticLimit = 256;
 
 struct FieldBuild {
   const float4* statics;  // WG poses
@@ -150,6 +155,36 @@ void fit_capsule(const std::vector<Ball>& balls, float* out) {
 
 }  // namespace
 
+// Whether every number of the plant's geometry is one the tables are made for:
+// finite, radii and half extents not negative, statics within
+// kFieldStaticLimit. Other plants keep the pair sweep.
+static bool ordinary_geometry(const HostPlant& hp, const std::vector<FkJoint>& fk) {
+  auto within = [](const float* v, int n, float lo, float hi) {
+    bool ok = true;
+    for (int i = 0; i < n; ++i) ok = ok && v[i] >= lo && v[i] <= hi;
+    return ok;
+  };
+  constexpr float kLim = (float)kFieldStaticLimit;
+  bool ok = true;
+  for (const FkJoint& j : fk)
+    ok = ok && within(j.P, 9, -4.f, 4.f) && within(j.S, 9, -4.f, 4.f) && within(j.T, 9, -4.f, 4.f) &&
+         within(j.t, 3, -kLim, kLim) && within(j.v, 3, -4.f, 4.f);
+  for (const MovingGeom& g : hp.moving)
+    ok = ok && within(g.p, 3, -kLim, kLim) && within(&g.r, 1, 0.f, kLim) &&
+         (g.type == G_SPHERE || (within(&g.hl, 1, 0.f, kLim) && within(g.z, 3, -2.f, 2.f)));
+  for (size_t s = 0; s < hp.static_type.size(); ++s) {
+    const float* W = hp.statics.data() + 16 * s;
+    if (hp.static_type[s] == G_SPHERE)
+      ok = ok && within(W, 3, -kLim, kLim) && within(W + 3, 1, 0.f, kLim);
+    else if (hp.static_type[s] == G_CAPSULE)
+      ok = ok && within(W, 3, -kLim, kLim) && within(W + 3, 1, 0.f, kLim) && within(W + 4, 3, -2.f, 2.f) &&
+           within(W + 7, 1, 0.f, kLim);
+    else
+      ok = ok && within(W, 12, -kLim, kLim) && within(W + 12, 3, 0.f, kLim);
+  }
+  return ok;
+}
+
 csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const std::vector<uint32_t>& moving_pairs,
                          const std::vector<uint32_t>& world_bits, const std::vector<float>& rounded,
                          const std::vector<double>& static_box, const std::vector<double>& reach_box) {
@@ -157,7 +192,8 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
   const HostPlant& hp = h->host;
   const int S = dp.num_static, M = dp.num_moving, NS = dp.num_slots;
   dp.has_field = 0;
-  if (!h->cull_eligible || M == 0 || M > 0xffff || S > kFieldMaxStatics || dp.num_msph + dp.num_mcap != M)
+  if (!h->cull_eligible || M == 0 || M > 0xffff || S > kFieldMaxStatics || dp.num_msph + dp.num_mcap != M ||
+      !ordinary_geometry(hp, fk))
     return CSD_OK;
   FieldTables f{};
   // ---- geometries, probes, link capsules
@@ -168,7 +204,6 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
     const MovingGeom& g = hp.moving[m];
     for (int k = 0; k < 3; ++k) geom[4 * m + k] = g.p[k];
     geom[4 * m + 3] = g.r;
-    if (!(g.r >= 0.f) || !(g.hl >= 0.f || g.type == G_SPHERE)) return CSD_OK;  // odd radii: the pair sweep decides
     if (g.type == G_SPHERE) {
       max_r = std::max(max_r, (double)g.r);
       balls[g.slot].push_back({{g.p[0], g.p[1], g.p[2]}, g.r});
@@ -296,8 +331,11 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
       const double pad = max_r * (1 + 1e-6) + 1e-3;
       f.far_lo[k] = (float)(static_box[k] - pad);
       f.far_hi[k] = (float)(static_box[3 + k] + pad);
-      lo[k] = std::max((double)f.far_lo[k], reach_box[k]);
-      hi[k] = std::max(lo[k] + 1e-3, std::min((double)f.far_hi[k], reach_box[3 + k]));
+      // (a prismatic joint's reach has no bound: its grid ends at the limit, and probes beyond test every static)
+      lo[k] = std::max((double)f.far_lo[k], reach_box[k] < -1e299 ? -kFieldGridLimit : reach_box[k]);
+      hi[k] = std::max(lo[k] + 1e-3,
+                       std::min((double)f.far_hi[k], reach_box[3 + k] > 1e299 ? kFieldGridLimit : reach_box[3 + k]));
+      if (lo[k] < -kFieldGridLimit || hi[k] > kFieldGridLimit) return CSD_OK;
       vol *= hi[k] - lo[k];
     }
     double edge = std::max(std::cbrt(vol / kFieldCells), kFieldMinEdge);
