@@ -17,6 +17,7 @@ constexpr int kFieldMaxStatics = 1024;   // as the broad phase (cull_eligible)
 constexpr double kFieldMinEdge = 0.02;   // finer cells list the same statics
 constexpr double kProbeGrowth = 1.2;     // a probe's radius over its capsule's, at most (more probes below it)
 constexpr int kMaxProbes = 12;           // probes of one capsule
+constexpr size_t kFieldStaticShared = 2048;  // static shared memory of a checking kernel, at most (a plant, work items)
 // Largest coordinates (metres from the world's origin) of a grid's box and of a
 // static's extents: up to there the FP32 rounding of a probe's place in its cell
 // (4 ulp of 128 m on each axis) and of a distance to a static (2 ulp of 256 m)
@@ -324,6 +325,17 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
   }
   f.fk_steps = (int)steps.size() / f.fk_branches;
   f.fk_batch = std::min(kFkBatch / f.fk_branches, dp.num_slots <= 8 ? 8 : dp.num_slots <= 16 ? 4 : 2);
+  // a block's warps have to fit: fewer configurations at once (their slot transforms are most of what the pair
+  // sweep does not need), or the pair sweep
+  int shared = 0;
+  CSD_CUDA_TRY(cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+  auto fits = [&] {
+    DevPlant t = dp;
+    t.field = f;
+    return (size_t)field_warp_floats(t) * sizeof(float) * kWarpsPerBlock + kFieldStaticShared <= (size_t)shared;
+  };
+  while (f.fk_batch > 1 && !fits()) f.fk_batch /= 2;
+  if (!fits()) return CSD_OK;
   // ---- grid over the part of the padded statics' box that the robot reaches
   if (S > 0) {
     double lo[3], hi[3], vol = 1;

@@ -98,3 +98,23 @@ def test_verdicts_far_from_the_origin(prismatic, base):
     on, off = on_off(plant, q)
     np.testing.assert_array_equal(on, off)
     assert 0 < off.mean() < 1
+
+
+# a block's eight warps hold the poses of up to some 1,780 moving spheres; the field path's batch of configurations
+# shrinks, and ends in the pair sweep, before they stop fitting
+@pytest.mark.parametrize("spheres", [1200, 1500, 1560, 1600, 1640, 1700, 1750])
+def test_plants_up_to_the_shared_memory_limit(spheres):
+    rng = np.random.default_rng(spheres)
+    more = [(S, tuple(rng.uniform(-0.1, 0.1, 3)), rng.uniform(0.01, 0.03)) for _ in range(spheres)]
+    plant = arm(ORDINARY[:2], moving=more)
+    pairs = plant.collision_pair_matrix()
+    assert plant.num_scene_geometries == spheres + 5
+    q = rng.uniform(-3, 3, (3001, 3)).astype(np.float32)
+    on, off = on_off(plant, q)
+    np.testing.assert_array_equal(on, off)
+    assert 0 < on.mean() < 1 and pairs.shape[1] > spheres
+    h = csd.plant_handle(plant)
+    s, e = np.ascontiguousarray(q[:64].T), np.ascontiguousarray(np.roll(q, 1, 0)[:64].T)
+    on = csd.CheckEdgesCollisionFreeCuda(s, e, plant, 0.05)
+    h.set_culling(False)
+    np.testing.assert_array_equal(on, csd.CheckEdgesCollisionFreeCuda(s, e, plant, 0.05))
