@@ -14,6 +14,7 @@ namespace {
 
 constexpr int kFieldCells = 1 << 18;     // most cells of a grid (16 bytes each)
 constexpr int kFieldMaxStatics = 1024;   // as the broad phase (cull_eligible)
+constexpr size_t kFieldMinList = 1 << 16; // entries of the cells' lists, at least (one cell can list kFieldMaxStatics)
 constexpr double kFieldMinEdge = 0.02;   // finer cells list the same statics
 constexpr double kProbeGrowth = 1.2;     // a probe's radius over its capsule's, at most (more probes below it)
 constexpr int kMaxProbes = 12;           // probes of one capsule
@@ -93,13 +94,11 @@ __global__ void __launch_bounds__(256) field_cells_kernel(FieldBuild b) {
   }
   if (cnt > 6) {
     const unsigned at = atomicAdd(b.used, (unsigned)cnt);
-    if (at + (unsigned)cnt <= b.list_cap && cnt < kFieldAll) {
+    if (at + (unsigned)cnt <= b.list_cap) {  // (otherwise the host builds again with fewer cells)
       unsigned j = at;
       for (int k = 0; k < num_near; ++k)
         if (!(static_distance(b, near[k], c) > b.reach)) b.list[j++] = near[k];
       w[0] = at;
-    } else {
-      cnt = kFieldAll;  // no room for the list: the cell tests every static
     }
   }
   // padded (the FP32 distances are off by far less) and rounded down
@@ -337,22 +336,10 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
   while (f.fk_batch > 1 && !fits()) f.fk_batch /= 2;
   if (!fits()) return CSD_OK;
   // ---- grid over the part of the padded statics' box that the robot reaches
-  if (S > 0) {
-    double lo[3], hi[3], vol = 1;
-    for (int k = 0; k < 3; ++k) {
-      const double pad = max_r * (1 + 1e-6) + 1e-3;
-      f.far_lo[k] = (float)(static_box[k] - pad);
-      f.far_hi[k] = (float)(static_box[3 + k] + pad);
-      // (a prismatic joint's reach has no bound: its grid ends at the limit, and probes beyond test every static)
-      lo[k] = std::max((double)f.far_lo[k], reach_box[k] < -1e299 ? -kFieldGridLimit : reach_box[k]);
-      hi[k] = std::max(lo[k] + 1e-3,
-                       std::min((double)f.far_hi[k], reach_box[3 + k] > 1e299 ? kFieldGridLimit : reach_box[3 + k]));
-      if (lo[k] < -kFieldGridLimit || hi[k] > kFieldGridLimit) return CSD_OK;
-      vol *= hi[k] - lo[k];
-    }
-    double edge = std::max(std::cbrt(vol / kFieldCells), kFieldMinEdge);
+  double lo[3], hi[3], edge = 0;
+  auto set_grid = [&](double e) {  // cells of edge e or the least larger one that keeps their number
     int n[3];
-    for (;; edge *= 1.01) {
+    for (edge = e;; edge *= 1.01) {
       for (int k = 0; k < 3; ++k) n[k] = (int)std::min(1e6, std::ceil((hi[k] - lo[k]) / edge));
       if ((double)n[0] * n[1] * n[2] <= kFieldCells) break;
     }
@@ -364,13 +351,28 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
     f.nx = n[0];
     f.ny = n[1];
     f.nz = n[2];
+  };
+  if (S > 0) {
+    double vol = 1;
+    for (int k = 0; k < 3; ++k) {
+      const double pad = max_r * (1 + 1e-6) + 1e-3;
+      f.far_lo[k] = (float)(static_box[k] - pad);
+      f.far_hi[k] = (float)(static_box[3 + k] + pad);
+      // (a prismatic joint's reach has no bound: its grid ends at the limit, and probes beyond test every static)
+      lo[k] = std::max((double)f.far_lo[k], reach_box[k] < -1e299 ? -kFieldGridLimit : reach_box[k]);
+      hi[k] = std::max(lo[k] + 1e-3,
+                       std::min((double)f.far_hi[k], reach_box[3 + k] > 1e299 ? kFieldGridLimit : reach_box[3 + k]));
+      if (lo[k] < -kFieldGridLimit || hi[k] > kFieldGridLimit) return CSD_OK;
+      vol *= hi[k] - lo[k];
+    }
+    set_grid(std::max(std::cbrt(vol / kFieldCells), kFieldMinEdge));
   }
   bool all = true;
   f.pair_words = (S + 31) / 32;
   for (int m = 0; m < M && all; ++m)
     for (int s = 0; s < S; ++s) all = all && ((world_bits[(size_t)m * f.pair_words + (s >> 5)] >> (s & 31)) & 1u);
   // ---- upload
-  const size_t cells = (size_t)f.nx * f.ny * f.nz, list_cap = std::max<size_t>(8 * cells, 16);
+  const size_t cells = (size_t)f.nx * f.ny * f.nz, list_cap = std::max<size_t>(8 * cells, kFieldMinList);
   size_t off = 0;
   auto section = [&](size_t bytes) {
     const size_t o = off;
@@ -419,29 +421,44 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
     b.statics = dp.statics;
     b.type = dp.static_type;
     b.S = S;
-    b.ox = f.ox;
-    b.oy = f.oy;
-    b.oz = f.oz;
-    b.h = f.h;
-    b.nx = f.nx;
-    b.ny = f.ny;
-    b.nz = f.nz;
-    const double half = 0.5 * std::sqrt(3.0) * f.h;
-    b.reach = (float)((max_r + half) * (1 + 1e-5) + 3e-4);
-    b.cap = (float)(max_r + half + 2.5e-4);
     b.cells = (uint4*)(base + o_cells);
     b.list = (uint16_t*)(base + o_list);
     b.list_cap = (unsigned)list_cap;
     b.used = (unsigned*)(base + o_used);
-    const dim3 grid((f.nx + 7) / 8, (f.ny + 7) / 8, (f.nz + 3) / 4);
-    if (grid.y > 65535u || grid.z > 65535u) {  // a sliver of a box: not worth a grid
+    auto keep_sweep = [&] {
       cudaFree(h->field_blob);
       h->field_blob = nullptr;
       return CSD_OK;
+    };
+    for (bool first = true;; first = false) {
+      b.ox = f.ox;
+      b.oy = f.oy;
+      b.oz = f.oz;
+      b.h = f.h;
+      b.nx = f.nx;
+      b.ny = f.ny;
+      b.nz = f.nz;
+      const double half = 0.5 * std::sqrt(3.0) * f.h;
+      b.reach = (float)((max_r + half) * (1 + 1e-5) + 3e-4);
+      b.cap = (float)(max_r + half + 2.5e-4);
+      const dim3 grid((f.nx + 7) / 8, (f.ny + 7) / 8, (f.nz + 3) / 4);
+      if (grid.y > 65535u || grid.z > 65535u) return keep_sweep();  // a sliver of a box: not worth a grid
+      field_cells_kernel<<<grid, 256>>>(b);
+      CSD_CUDA_TRY(cudaGetLastError());
+      // (the copy waits for the kernel: the tables are read from any stream after this)
+      unsigned used = 0;
+      CSD_CUDA_TRY(cudaMemcpy(&used, b.used, sizeof(used), cudaMemcpyDeviceToHost));
+      // One probe much larger than the others makes every list long. Up to about S / 25 entries a cell the field path
+      // is the faster (131,072 configurations of an arm with one sphere of 0.3 to 1 m among 900, 300 and 100 small
+      // statics: 1.0 -> 0.4 ms against the pair sweep with 26 entries, 1.0 -> 1.2 with 50; 0.54 -> 0.26 with 8,
+      // 0.54 -> 0.61 with 16; 0.34 -> 0.25 with 4, 0.35 -> 0.46 with 7).
+      if (first && used > (2.0 + S / 25.0) * cells) return keep_sweep();
+      if (used <= list_cap) break;
+      // The lists do not fit. Wider cells list little more each (the large probe's radius decides), so fewer of them
+      // do; with cells without room testing every static those arms took 3.7 to 5.5 ms.
+      set_grid(1.03 * edge * std::cbrt((double)used / list_cap));
+      CSD_CUDA_TRY(cudaMemset(b.used, 0, sizeof(used)));
     }
-    field_cells_kernel<<<grid, 256>>>(b);
-    CSD_CUDA_TRY(cudaGetLastError());
-    CSD_CUDA_TRY(cudaDeviceSynchronize());  // the tables are read from any stream after this
   }
   dp.field = f;
   dp.has_field = 1;
