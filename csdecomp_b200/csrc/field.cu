@@ -4,7 +4,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
 
 #include "check_field.cuh"
 
@@ -239,29 +238,23 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
     else
       fit_capsule(balls[k], &link[8 * k]);
   }
-  // ---- moving-moving pairs by link pair, then by type
-  std::map<std::pair<int, int>, std::vector<uint32_t>> by_link[3];
-  std::map<std::pair<int, int>, int> keys;
-  for (uint32_t w : moving_pairs) {
-    const int a = (int)(w & 0xffffu), b = (int)(w >> 16);
-    const int ty = (hp.moving[a].type == G_CAPSULE) + (hp.moving[b].type == G_CAPSULE);
-    std::pair<int, int> key(hp.moving[a].slot, hp.moving[b].slot);
-    if (key.first > key.second) std::swap(key.first, key.second);
-    by_link[ty][key].push_back(w);
-    keys[key] = 1;
-  }
+  // ---- moving-moving pairs by link pair, then by type, in the order given (a counting sort: a tree of vectors cost
+  // plant creation 0.2 to 0.4 ms for some 3,000 pairs)
+  auto bucket = [&](uint32_t w) {
+    const MovingGeom &a = hp.moving[w & 0xffffu], &b = hp.moving[w >> 16];
+    const int ty = (a.type == G_CAPSULE) + (b.type == G_CAPSULE);
+    return (std::min(a.slot, b.slot) * NS + std::max(a.slot, b.slot)) * 3 + ty;
+  };
+  std::vector<int> begin((size_t)NS * NS * 3 + 1, 0);
+  for (uint32_t w : moving_pairs) ++begin[bucket(w) + 1];
+  for (size_t k = 1; k < begin.size(); ++k) begin[k] += begin[k - 1];
   std::vector<LinkPair> lps;
-  std::vector<uint32_t> pairs;
-  for (auto& kv : keys) {
-    LinkPair lp{kv.first.first, kv.first.second, (int)pairs.size(), 0, 0, 0};
-    int* n[3] = {&lp.nss, &lp.nsc, &lp.ncc};
-    for (int ty = 0; ty < 3; ++ty) {
-      const std::vector<uint32_t>& v = by_link[ty][kv.first];
-      *n[ty] = (int)v.size();
-      pairs.insert(pairs.end(), v.begin(), v.end());
-    }
-    lps.push_back(lp);
+  for (int k = 0; k < NS * NS; ++k) {
+    const int* o = &begin[3 * k];
+    if (o[3] > o[0]) lps.push_back({k / NS, k % NS, o[0], o[1] - o[0], o[2] - o[1], o[3] - o[2]});
   }
+  std::vector<uint32_t> pairs(moving_pairs.size());
+  for (uint32_t w : moving_pairs) pairs[begin[bucket(w)]++] = w;
   // ---- FK table
   std::vector<float> entry((size_t)dp.num_fk * 36, 0.f);
   for (int j = 0; j < dp.num_fk; ++j)
