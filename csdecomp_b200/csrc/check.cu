@@ -304,15 +304,56 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n)
 }
 
 // ---------------------------------------------------------------- FK output
-// All link transforms as column-major 4x4. Lane per configuration: a lane
-// walks the tree with one slot transform in registers (those that joints
-// branch off from later are kept in the warp's shared memory), so every lane
-// works and no value crosses lanes. After each joint the links on its slot
-// (listed by slot) are composed and written through a shared tile, four lanes
-// per matrix, whole 32-byte sectors. The output is the work: 64 bytes per
-// link. A warp per configuration (12 of 32 lanes composing by shuffles, each
-// matrix stored as four 16-byte pieces per lane) reached 0.7 TB/s: 87 us for
-// 100,003 configurations of 9 links, 16 us here (3.7 TB/s).
+// All link transforms as column-major 4x4, by one of two kernels (launch_fk).
+
+// Warp per configuration: FK as the checks run it, then lane l composes and
+// writes links l, l + 32, ... Its latency is one configuration's, so it serves
+// small batches, and it stages nothing per link, so it serves any tree.
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) fk_warp_kernel(DevPlant p, const float* __restrict__ q, int64_t n,
+                                                                     float* __restrict__ tf_out) {
+  extern __shared__ float4 smem4[];
+  const int lane = threadIdx.x & 31;
+  float* X = reinterpret_cast<float*>(smem4) + (threadIdx.x >> 5) * (p.num_slots * 12 + kMaxDim);
+  float* qs = X + p.num_slots * 12;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += nw) {
+    if (lane < p.dim) qs[lane] = q[i * p.dim + lane];
+    __syncwarp();
+    fk_warp(p, qs, X, lane);
+    __syncwarp();
+    for (int l = lane; l < p.num_links; l += kWarp) {
+      const int s = __ldg(p.link_slot + l);
+      const float4* F = reinterpret_cast<const float4*>(p.link_fixed + 12 * l);
+      const float4 a = __ldg(F), b = __ldg(F + 1), c = __ldg(F + 2);
+      const float Rf[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x}, tf[3] = {c.y, c.z, c.w};
+      float R[9], t[3];
+      if (s < 0) {  // welded to the world, or unreachable (zeros)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) R[k] = s == -1 ? Rf[k] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) t[k] = s == -1 ? tf[k] : 0.f;
+      } else {
+        compose(X + s * 12, X + s * 12 + 9, Rf, tf, R, t);
+      }
+      float4* dst = reinterpret_cast<float4*>(tf_out + (i * p.num_links + l) * 16);
+      dst[0] = make_float4(R[0], R[1], R[2], 0.f);
+      dst[1] = make_float4(R[3], R[4], R[5], 0.f);
+      dst[2] = make_float4(R[6], R[7], R[8], 0.f);
+      dst[3] = make_float4(t[0], t[1], t[2], s == -2 ? 0.f : 1.f);
+    }
+    __syncwarp();
+  }
+}
+
+// Lane per configuration: a lane walks the tree with one slot transform in
+// registers (those that joints branch off from later are kept in the warp's
+// shared memory), so every lane works and no value crosses lanes. After each
+// joint the links on its slot (link_order lists them by slot) are composed and
+// written through a shared tile, four lanes per matrix, whole 32-byte sectors.
+// The output is the work: 64 bytes per link. fk_warp_kernel (12 of 32 lanes
+// composing by shuffles, each matrix stored as four 16-byte pieces per lane)
+// reaches 0.7 TB/s: 87 us for 100,003 configurations of 9 links, 16 us here
+// (3.7 TB/s).
 constexpr int kFkWarps = 4;
 constexpr int kFkTile = kWarp * 20;  // floats: 32 matrices, rows padded against bank conflicts
 
@@ -340,12 +381,9 @@ __global__ void __launch_bounds__(kFkWarps * 32) fk_kernel(DevPlant p, const flo
   for (int i = threadIdx.x; i < p.num_fk * (int)(sizeof(FkJoint) / 4); i += blockDim.x)
     tab[i] = __ldg(reinterpret_cast<const float*>(p.fk) + i);
   for (int i = threadIdx.x; i < 12 * L; i += blockDim.x) fixed[i] = __ldg(p.link_fixed + i);
-  for (int i = threadIdx.x; i < L; i += blockDim.x) lslot[i] = __ldg(p.link_slot + i);
-  __syncthreads();
-  for (int i = threadIdx.x; i < L; i += blockDim.x) {  // links by slot: unreachable (-2), world (-1), 0, 1, ...
-    int r = 0;
-    for (int l = 0; l < L; ++l) r += lslot[l] < lslot[i] || (lslot[l] == lslot[i] && l < i);
-    order[r] = i;
+  for (int i = threadIdx.x; i < L; i += blockDim.x) {
+    lslot[i] = __ldg(p.link_slot + i);
+    order[i] = __ldg(p.link_order + i);
   }
   __syncthreads();
   const int64_t nw = (int64_t)gridDim.x * kFkWarps;
@@ -446,10 +484,26 @@ csd_status_t launch_check_points(const csd_plant_s* p, const float* q, int64_t n
   });
 }
 
+// The lane kernel once it has the warps to cover its latency, a walk over the
+// whole tree: from 6,144 configurations and 64 per link on, 16,384 at most, and
+// where its tables fit a block. Warp kernel against lane kernel: 8 links 10.2 /
+// 12.3 us at 512 configurations, 12.3 / 12.3 at 6,144, 31.6 / 13.1 at 32,768;
+// 57 links 12.3 / 24.6 at 512, 23.2 / 23.3 at 8,192, 57 / 33 at 32,768; 2,101
+// links 33 / 465 at one, 516 / 586 at 12,288, 705 / 586 at 16,384.
+constexpr int64_t kFkLaneMin = 6144, kFkLanePerLink = 64, kFkLaneMost = 16384;
+constexpr size_t kFkLaneShared = 220 * 1024;
+
 csd_status_t launch_fk(const csd_plant_s* p, const float* q, int64_t n, float* tf, cudaStream_t st) {
   if (n <= 0) return CSD_OK;
-  const size_t smem = ((size_t)fk_table_words(p->dp) + (size_t)fk_warp_words(p->dp) * kFkWarps) * sizeof(float);
+  size_t smem = ((size_t)fk_table_words(p->dp) + (size_t)fk_warp_words(p->dp) * kFkWarps) * sizeof(float);
   int grid = 0;
+  if (n < std::min(kFkLaneMost, kFkLaneMin + kFkLanePerLink * p->dp.num_links) || smem > kFkLaneShared) {
+    smem = (size_t)(p->dp.num_slots * 12 + kMaxDim) * kWarpsPerBlock * sizeof(float);
+    if (csd_status_t s = grid_for(fk_warp_kernel, smem, n, &grid, kWarpsPerBlock)) return s;
+    fk_warp_kernel<<<grid, 32 * kWarpsPerBlock, smem, st>>>(p->dp, q, n, tf);
+    CSD_CUDA_TRY(cudaGetLastError());
+    return CSD_OK;
+  }
   if (csd_status_t s = grid_for(fk_kernel, smem, (n + kWarp - 1) / kWarp, &grid, kFkWarps)) return s;
   fk_kernel<<<grid, 32 * kFkWarps, smem, st>>>(p->dp, q, n, tf);
   CSD_CUDA_TRY(cudaGetLastError());

@@ -103,7 +103,7 @@ struct FieldTables {
   // max_r + half a cell diagonal (padded) of its centre: no other static can
   // touch a probe of radius <= max_r whose centre lies in the cell.
   const uint4* cells;       // x: distance of the centre to the nearest listed static (binary16, rounded down,
-                            // capped) | number of statics << 16 (0xffff: test every static); y, z, w: up to
+                            // capped) | number of statics << 16; y, z, w: up to
                             // six 16-bit static indices, or (more than six) y = first entry of `list`
   const uint16_t* list;     // indices of the cells with more than six statics
   float ox, oy, oz;         // corner of the grid
@@ -165,6 +165,7 @@ struct DevPlant {
   const GenSeg* segs;
   const PairRun* runs;
   const int* link_slot;        // [num_links] slot of each reference link (-1 world, -2 unreachable)
+  const int* link_order;       // [num_links] links by slot (unreachable, world, slot 0, 1, ...), ascending within one
   const float* link_fixed;     // [num_links][12] slot->link (R col-major 9, t 3); world links: world pose
   int* status;                 // device error word: nonzero after a bounded wait gave up
   int has_field;               // the field tables exist (used while `cull` is on)

@@ -872,7 +872,11 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
   size_t o_sg = section(segs.size() * sizeof(GenSeg));
   size_t o_ru = section(runs.size() * sizeof(PairRun));
   size_t o_status = section(16);
+  std::vector<int> link_order(L);
+  for (int l = 0; l < L; ++l) link_order[l] = l;
+  std::stable_sort(link_order.begin(), link_order.end(), [&](int x, int y) { return link_slot[x] < link_slot[y]; });
   size_t o_ls = section(link_slot.size() * sizeof(int));
+  size_t o_lo = section(link_order.size() * sizeof(int));
   size_t o_lf = section(link_fixed.size() * sizeof(float));
   std::vector<char> host_blob(off, 0);
   auto put = [&](size_t o, const void* src, size_t n) {
@@ -899,6 +903,7 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
   put(o_sg, segs.data(), segs.size() * sizeof(GenSeg));
   put(o_ru, runs.data(), runs.size() * sizeof(PairRun));
   put(o_ls, link_slot.data(), link_slot.size() * sizeof(int));
+  put(o_lo, link_order.data(), link_order.size() * sizeof(int));
   put(o_lf, link_fixed.data(), link_fixed.size() * sizeof(float));
   CSD_CUDA_TRY(cudaMalloc(&h->blob, off));
   CSD_CUDA_TRY(cudaMemcpy(h->blob, host_blob.data(), off, cudaMemcpyHostToDevice));
@@ -944,6 +949,7 @@ csd_status_t csd_plant_create(const csd_plant_desc_t* d, csd_plant_t* out) {
   dp.runs = (const PairRun*)(base + o_ru);
   dp.status = (int*)(base + o_status);
   dp.link_slot = (const int*)(base + o_ls);
+  dp.link_order = (const int*)(base + o_lo);
   dp.link_fixed = (const float*)(base + o_lf);
   if (csd_status_t s = build_field(h.get(), fk, moving_pairs, world_bits, rounded, static_box, reach_box)) return s;
   *out = h.release();
