@@ -431,9 +431,26 @@ static __device__ __forceinline__ bool field_voxels(const DevPlant& p, const flo
         n[k] = vox_cell(c[k] + fmaxf(R - va.grins, 0.f), va.ginv_h) - lo[k] + 1;
       }
       const bool finite = isfinite(c[0]) && isfinite(c[1]) && isfinite(c[2]) && isfinite(R);
-      if (!finite || (long long)n[0] * n[1] * n[2] > kVoxGridMaxCells) {  // (a NaN pose collides with every voxel)
-        for (int v = 0; v < va.nv && !hit; ++v)
-          hit = exact(__ldg(va.vox + 3 * v), __ldg(va.vox + 3 * v + 1), __ldg(va.vox + 3 * v + 2));
+      if (!finite || vox_sweep((long long)n[0] * n[1], n[2], va.nv)) {  // (a NaN pose collides with every voxel)
+        if (!cap) {  // four at a time, their loads together
+          const float A[4] = {c[0], c[1], c[2], r};
+          for (int v0 = 0; v0 < va.nv && !hit; v0 += 4) {
+            float S[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float* v = va.vox + 3 * min(v0 + j, va.nv - 1);
+              S[j][0] = __ldg(v);
+              S[j][1] = __ldg(v + 1);
+              S[j][2] = __ldg(v + 2);
+              S[j][3] = va.vr;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) hit = sph_sph_hit(A, S[j]) || hit;
+          }
+        } else {
+          for (int v = 0; v < va.nv && !hit; ++v)
+            hit = exact(__ldg(va.vox + 3 * v), __ldg(va.vox + 3 * v + 1), __ldg(va.vox + 3 * v + 2));
+        }
       } else {
         cols = n[0] * n[1];
       }
