@@ -29,6 +29,16 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n)
   if (!w.ok) return;
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  if constexpr (M != kModeField) {
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += nw) {
+      if (lane < p.dim) w.qs[lane] = q[i * p.dim + lane];
+      __syncwarp();
+      fk_warp(p, w.qs, w.X, lane);
+      const bool hit = check_config(p, w.stat, w.aabb, w.X, w.pose, lane, va);
+      if (lane == 0) out[i] = hit ? 0 : 1;
+    }
+    return;
+  }
   // runs of a warp's batch, shorter when there are not enough configurations for every warp
   const int64_t per = (n + nw - 1) / nw;
   const int64_t B = per < warp_batch<M>(p) ? per : warp_batch<M>(p);
@@ -157,6 +167,25 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, ModeBlocks<M>::n) check_e
     const int64_t G = (np + 31) / 32;
     bool collided = false;
     int64_t checked = 0;
+    if constexpr (M != kModeField) {
+      const float a1 = lane < d ? w.q1[lane] : 0.f, a2 = lane < d ? w.q2[lane] : 0.f;
+      for (int64_t v = 0; v < 32 * G && !collided; ++v) {
+        const int64_t k = (v % 32) * G + v / 32;
+        if (k >= np) continue;
+        const float x = edge_coord(a1, a2, np, mode, k);
+        __syncwarp();
+        if (lane < d) w.qs[lane] = x;
+        __syncwarp();
+        fk_warp(p, w.qs, w.X, lane);
+        ++checked;
+        collided = check_config(p, w.stat, w.aabb, w.X, w.pose, lane, none);
+      }
+      if (lane == 0) {
+        out[e] = collided ? 0 : 1;
+        if (pts) pts[e] = checked;
+      }
+      continue;
+    }
     // batches of visits share their FK; a visit past the edge's points repeats the last point and is not checked
     const int B = warp_batch<M>(p);
     for (int64_t v0 = 0; v0 < 32 * G && !collided; v0 += B) {

@@ -89,6 +89,17 @@ static __device__ __forceinline__ bool check_nth(const DevPlant& p, const WarpCt
 template <int M, typename F>
 static __device__ __forceinline__ void check_range(const DevPlant& p, const WarpCtx<M>& w, const float* __restrict__ q,
                                                    int64_t i0, int64_t i1, int lane, const VoxArgs& va, F verdict) {
+  if constexpr (M != kModeField) {
+    for (int64_t i = i0; i < i1; ++i) {
+      __syncwarp();
+      if (lane < p.dim) w.qs[lane] = q[i * p.dim + lane];
+      __syncwarp();
+      fk_warp(p, w.qs, w.X, lane);
+      const bool hit = check_config(p, w.stat, w.aabb, w.X, w.pose, lane, va);
+      if (lane == 0) verdict(i, hit);
+    }
+    return;
+  }
   const int B = warp_batch<M>(p);
   for (int64_t i = i0; i < i1; i += B) {
     const int m = (int)(i1 - i < B ? i1 - i : B);

@@ -69,6 +69,47 @@ static __device__ __forceinline__ void bisect_particles(const DevPlant& p, const
                                                         int steps, S0 starts, S1 ends, const VoxArgs& va,
                                                         float* __restrict__ cols, float* __restrict__ proj,
                                                         float* __restrict__ dist, int lane) {
+  if constexpr (M != kModeField) {  // one particle (m is 1)
+    const float* ci = cols + (size_t)i0 * dim;
+    const float *ls = starts(i0), *le = ends(i0);
+    float seg2 = 0.f, a = 0.f;
+    for (int k = 0; k < dim; ++k) {
+      float dk = __fsub_rn(le[k], ls[k]);
+      seg2 = __fmaf_rn(dk, dk, seg2);
+      a = __fmaf_rn(__fsub_rn(ci[k], ls[k]), dk, a);
+    }
+    const float t = fminf(fmaxf(__fdiv_rn(a, seg2), 0.0f), 1.0f);
+    const float omt = __fsub_rn(1.0f, t);
+    float pr = 0.f, lo = 0.f, hi = 0.f;
+    if (lane < dim) {
+      pr = __fmaf_rn(t, le[lane], __fmul_rn(omt, ls[lane]));
+      lo = pr;
+      hi = ci[lane];
+    }
+    for (int s = 0; s < steps; ++s) {
+      const float mid = __fmul_rn(0.5f, __fadd_rn(lo, hi));
+      __syncwarp();
+      if (lane < dim) w.qs[lane] = mid;
+      __syncwarp();
+      fk_warp(p, w.qs, w.X, lane);
+      if (check_config(p, w.stat, w.aabb, w.X, w.pose, lane, va))
+        hi = mid;
+      else
+        lo = mid;
+    }
+    __syncwarp();
+    if (lane < dim) w.qs[lane] = __fsub_rn(hi, pr);
+    __syncwarp();
+    float s2 = 0.f;
+    for (int k = 0; k < dim; ++k) s2 = __fmaf_rn(w.qs[k], w.qs[k], s2);
+    if (lane < dim) {
+      cols[(size_t)i0 * dim + lane] = hi;
+      proj[(size_t)i0 * dim + lane] = pr;
+    }
+    if (lane == 0) dist[i0] = __fsqrt_rn(s2);
+    __syncwarp();
+    return;
+  }
   constexpr int MB = M == kModeField ? kFkBatch : 1;
   float lo[MB], hi[MB];  // hi: the collision point so far
 #pragma unroll
