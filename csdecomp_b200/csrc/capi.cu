@@ -433,7 +433,7 @@ csd_status_t csd_uniform_sample_hpolyhedra(const float* A, const float* b, const
   if (!s && cudaMemsetAsync(pnf, 0, sizeof(int), st) != cudaSuccess) s = CSD_ERR_CUDA;
   if (!s)
     s = launch_hit_and_run((const float*)pA, (const float*)pb, (const int32_t*)po, P, dim, (const float*)ps, S, mixing,
-                           seed, (float*)pout, pnf, st);
+                           seed, (float*)pout, pnf, st, face_off);
   int nf = 0;
   if (!s && (cudaMemcpyAsync(samples, pout, bout, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
              cudaMemcpyAsync(&nf, pnf, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

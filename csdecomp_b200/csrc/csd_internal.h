@@ -195,7 +195,7 @@ csd_status_t launch_check_edges_ranked(const csd_plant_s* p, const float* s0, co
 // sampler.cu
 csd_status_t launch_hit_and_run(const float* A, const float* b, const int32_t* face_off, int num_poly, int dim,
                                 const float* starts, int samples_per_poly, int mixing, uint64_t seed, float* out,
-                                int* num_failed, cudaStream_t st);
+                                int* num_failed, cudaStream_t st, const int32_t* face_off_host = nullptr);
 // EI-ZO sampler over one region stored as face-pair rows (sampler_core.cuh,
 // pair_stride(dim) floats per row, start slacks at `start`); the face count is
 // read on the device. A failed chain keeps its start point.
