@@ -63,6 +63,7 @@ struct BatchIter {    // device-side iteration state
   int num_act;        // length of the active-slot list of iteration k
   int max_nf8;        // most faces of an active slot with dim <= 8
   int max_nf16;       // most faces of an active slot with dim > 8 (of those not sampled from registers)
+  int all_nf16;       // most faces of any active slot with dim > 8
   int sample_next;    // work queues of the sampler, check and bisection launches: items claimed past the
   int check_next;     // first one per block (each zeroed before every launch that uses it)
   int bisect_next;
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(256, MINB) batch_sample_kernel(BatchArgs a, in
 // from the queue it->reg_next: the face pairs in registers
 // (sample_region_regs), or as batch_sample_kernel<8, 1> for a slot of another
 // size. One block per SM: four pairs of 14 coordinates and four chains' slacks
-// and dot products take 240 registers a thread.
+// and dot products fill the 255 registers of a thread.
 __global__ void __launch_bounds__(256, 1) batch_sample_regs_kernel(BatchArgs a, int all) {
   extern __shared__ __align__(16) float smf[];
   __shared__ GroupScratch gsa[kMaxWideGroups];
@@ -416,13 +417,14 @@ __global__ void __launch_bounds__(1024) batch_faces_kernel(BatchArgs a) {
 // from registers first, then the others, each part ascending.
 __global__ void __launch_bounds__(1024) batch_step_kernel(BatchArgs a) {
   __shared__ int warp_n[2][32];
-  __shared__ int base[2], nreg, mf8, mf16, nord, nmax, nfin;
+  __shared__ int base[2], nreg, mf8, mf16, all16, nord, nmax, nfin;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   if (tid == 0) {
     base[0] = 0;
     nreg = 0;
     mf8 = 0;
     mf16 = 0;
+    all16 = 0;
     nord = 0;
     nmax = 0;
     nfin = 0;
@@ -437,6 +439,7 @@ __global__ void __launch_bounds__(1024) batch_step_kernel(BatchArgs a) {
         atomicAdd(&nreg, 1);
       else
         atomicMax(S.dim <= 8 ? &mf8 : &mf16, S.nf);
+      if (S.dim > 8) atomicMax(&all16, S.nf);
       atomicMax(&nmax, a.n_tab[min(S.k, a.max_iters - 1)]);
       if (S.ord) atomicAdd(&nord, 1);
     } else if (!S.harvested) {
@@ -474,6 +477,7 @@ __global__ void __launch_bounds__(1024) batch_step_kernel(BatchArgs a) {
     it->num_reg = nreg;
     it->max_nf8 = mf8;
     it->max_nf16 = mf16;
+    it->all_nf16 = all16;
     it->num_ord = nord;
     it->n_act = nmax;
     it->num_fin = nfin;
@@ -782,7 +786,8 @@ struct csd_batch_s {
   int run_variant = 0;        // variant of the current iterations
   bool switch_large = true;   // false after csd_batch_set_shapes: run exactly the set variant
   int sample_grid[csd::kNumSampleVariants] = {};
-  int tune_iters = 0;                               // iterations of the next inflate to tune on
+  int tune_iters = 0;                               // iterations left to time check item sizes on
+  int tune_samples = 0;                             // iterations left to time sampler variants on (staged samplers only)
   double tune_ms[csd::kNumSampleVariants + csd::kNumCheckVariants] = {};
   int tuned_iters = 0;
   // large regions: the first time a region outgrows the tuned variant's staging, the next
@@ -1298,7 +1303,11 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
   int active_now = ns;
   for (;;) {
     const int samplers = samplers_needed(*h->host_iter);
-    if (h->large_pending && h->tune_iters == 0) {
+    // the sampler variants are timed on iterations that run the staged sampler: beside the register sampler alone
+    // they would find nothing to do
+    const bool staged = (samplers & kSampleStaged) != 0;
+    const bool tune_check = h->tune_iters > 0, tune_sample = h->tune_samples > 0 && staged;
+    if (h->large_pending && staged && !tune_check && !tune_sample) {
       // regions outgrew the tuned variant's staging for the first time: every sampler variant
       // on this iteration's inputs (the stage is idempotent), then the rest of the iteration;
       // the fastest samples the large regions from here on
@@ -1329,7 +1338,7 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
       if (h->profile)
         CSD_CUDA_TRY(cudaMemcpyAsync(prof_slots.data(), h->slots_dev.ptr, ns * sizeof(SlotState),
                                      cudaMemcpyDeviceToHost, st));
-    } else if (h->tune_iters > 0) {
+    } else if (tune_check || tune_sample) {
       // every sampler variant and check item size on this iteration's inputs
       // (both stages are idempotent: a rerun writes the same samples and
       // verdicts), then the rest of the iteration as usual
@@ -1337,15 +1346,16 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
         for (cudaEvent_t& e : h->ev) CSD_CUDA_TRY(cudaEventCreate(&e));
       std::vector<cudaEvent_t> tev(2 * (kNumSampleVariants + kNumCheckVariants));
       for (cudaEvent_t& e : tev) CSD_CUDA_TRY(cudaEventCreate(&e));
-      int j = 0;
-      for (int v = 0; v < kNumSampleVariants; ++v, ++j) {
+      for (int v = 0; v < kNumSampleVariants && tune_sample; ++v) {
         cudaMemsetAsync(&a.it->sample_next, 0, sizeof(int), st);
-        cudaEventRecord(tev[2 * j], st);
+        cudaEventRecord(tev[2 * v], st);
         launch_staged_sampler(h, v, samplers, a, st);
-        cudaEventRecord(tev[2 * j + 1], st);
+        cudaEventRecord(tev[2 * v + 1], st);
         ++h->launches;
       }
-      for (int c = 0; c < kNumCheckVariants && !a.mlp_wb; ++c, ++j) {
+      const bool time_check = tune_check && !a.mlp_wb;
+      for (int c = 0; c < kNumCheckVariants && time_check; ++c) {
+        const int j = kNumSampleVariants + c;
         BatchArgs ac = a;
         ac.cfg_max = kCheckItemCaps[c];
         cudaMemsetAsync(&a.it->check_next, 0, sizeof(int), st);
@@ -1354,26 +1364,31 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
         cudaEventRecord(tev[2 * j + 1], st);
         ++h->launches;
       }
-      h->launches += launch_iteration(h, ns, a, st, nullptr, samplers, samplers & ~kSampleStaged);
+      h->launches +=
+          launch_iteration(h, ns, a, st, nullptr, samplers, tune_sample ? samplers & ~kSampleStaged : samplers);
       CSD_CUDA_TRY(cudaGetLastError());
       CSD_CUDA_TRY(cudaStreamSynchronize(st));
-      for (int q = 0; q < j; ++q) {
+      for (int q = 0; q < kNumSampleVariants + kNumCheckVariants; ++q) {
+        if (!(q < kNumSampleVariants ? tune_sample : time_check)) continue;
         float ms = 0.f;
         cudaEventElapsedTime(&ms, tev[2 * q], tev[2 * q + 1]);
         h->tune_ms[q] += ms;
       }
       for (cudaEvent_t& e : tev) cudaEventDestroy(e);
       ++h->tuned_iters;
-      if (--h->tune_iters == 0) {
-        int bs = 0, bc = 0;
+      if (tune_sample && --h->tune_samples == 0) {
+        int bs = 0;
         for (int v = 1; v < kNumSampleVariants; ++v)
           if (h->tune_ms[v] < h->tune_ms[bs]) bs = v;
-        for (int c = 1; c < kNumCheckVariants; ++c)
-          if (h->tune_ms[kNumSampleVariants + c] < h->tune_ms[kNumSampleVariants + bc]) bc = c;
         h->sample_variant = bs;
         h->run_variant = bs;
         // reported until a region outgrows bs's staging: the variant that would take over then
         h->large_variant = variant_for(h, kSampleVariants[bs].f8 + 1, kSampleVariants[bs].f16 + 1);
+      }
+      if (tune_check && --h->tune_iters == 0) {
+        int bc = 0;
+        for (int c = 1; c < kNumCheckVariants; ++c)
+          if (h->tune_ms[kNumSampleVariants + c] < h->tune_ms[kNumSampleVariants + bc]) bc = c;
         if (!a.mlp_wb) h->cfg_max = kCheckItemCaps[bc];
         a.cfg_max = h->cfg_max;
       }
@@ -1456,14 +1471,18 @@ csd_status_t csd_batch_inflate(csd_batch_t h, int32_t n, const int32_t* slot_pla
     // a slot's region outgrew the staging buffer of the running variant: the first time, time
     // every variant on the next iteration; after that, continue with the fastest variant (by
     // those times) that stages it (identical samples; the graph is captured again)
-    if (h->switch_large && h->tune_iters == 0 && !h->large_pending) {
+    const int next = samplers_needed(*h->host_iter);
+    if (h->switch_large && (next & kSampleStaged) && h->tune_iters == 0 && h->tune_samples == 0 && !h->large_pending) {
       const SampleVariant& rv = kSampleVariants[h->run_variant];
-      if (h->host_iter->max_nf8 > rv.f8 || h->host_iter->max_nf16 > rv.f16) {
+      // without the register sampler the staged one takes every slot
+      const int nf8 = h->host_iter->max_nf8,
+                nf16 = next == kSampleStaged ? h->host_iter->all_nf16 : h->host_iter->max_nf16;
+      if (nf8 > rv.f8 || nf16 > rv.f16) {
         if (!h->large_tuned) {
           h->large_pending = true;
           continue;
         }
-        const int v = variant_for(h, h->host_iter->max_nf8, h->host_iter->max_nf16);
+        const int v = variant_for(h, nf8, nf16);
         if (v != h->run_variant) {
           h->run_variant = v;
           h->large_variant = v;
@@ -1518,6 +1537,7 @@ csd_status_t csd_batch_stage_ms(csd_batch_t h, float* ms) {
 csd_status_t csd_batch_autotune(csd_batch_t h, int32_t iterations) {
   CSD_CHECK(h && iterations >= 0, CSD_ERR_INVALID, "bad autotune arguments");
   h->tune_iters = iterations;
+  h->tune_samples = iterations;
   h->tuned_iters = 0;
   for (double& x : h->tune_ms) x = 0.0;
   h->large_tuned = false;
