@@ -92,7 +92,7 @@ EXPORTS = (
     "csd_batch_set_profiling", "csd_batch_stage_ms", "csd_batch_iteration_profile", "csd_batch_iteration_variants", "csd_batch_sample_flops", "csd_batch_last_launches",
     "csd_batch_autotune", "csd_batch_tuning", "csd_batch_set_shapes", "csd_batch_sample_variants", "csd_batch_shape_counts", "csd_batch_set_surrogate",
     "csd_batch_set_surrogate_rounds",    "csd_batch_destroy",
-    "csd_num_samples_unadaptive", "csd_fp32_fma_probe", "csd_plant_flops", "csd_plant_set_culling",
+    "csd_num_samples_unadaptive", "csd_fp32_fma_probe", "csd_quotient_probe", "csd_plant_flops", "csd_plant_set_culling",
     "csd_plant_set_voxel_grid",
     "csd_urdf_create", "csd_urdf_destroy", "csd_urdf_register_package", "csd_urdf_parse_file",
     "csd_urdf_parse_string", "csd_urdf_parse_directives", "csd_urdf_plant_desc", "csd_urdf_limits",

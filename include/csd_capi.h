@@ -455,6 +455,14 @@ uint32_t csd_num_samples_unadaptive(float epsilon, float delta, float tau);
 /* Diagnostics (no counterpart in the reference): FP32 FMA throughput of the
  * current device, the denominator of the collision kernels' roofline. */
 csd_status_t csd_fp32_fma_probe(int64_t iters, double* flops, double* seconds);
+/* Diagnostics (no counterpart in the reference): compares the samplers' packed
+ * quotient with the IEEE division bit for bit, numerators s[0..ns) by every
+ * divisor a[0..na) or, paired, s[i] by a[i] (host arrays of up to 2^24 floats).
+ * *mismatches: operand pairs whose quotients differ; example[2] (or NULL): one
+ * such numerator and divisor. They have to agree for numerators of at least
+ * 2^-30 and quotients of 2^-100 to 2^29 in magnitude. */
+csd_status_t csd_quotient_probe(const float* s, int64_t ns, const float* a, int64_t na, int32_t paired,
+                                int64_t* mismatches, float* example);
 /* Broad phase of the collision checks (no counterpart in the reference, which
  * tests every pair): pairs apart by more than 1e-4 m are skipped, found through
  * a grid over the statics and capsules around the links or, for plants with
