@@ -64,11 +64,6 @@ __device__ __forceinline__ int64_t edge_points(const float* q1, const float* q2,
   return (int64_t)(uint32_t)x;
 }
 
-__device__ __forceinline__ void lerp_point(const float* q1, const float* q2, int d, float t, float* out) {
-  float omt = __fsub_rn(1.0f, t);
-  for (int k = 0; k < d; ++k) out[k] = __fadd_rn(__fmul_rn(t, q2[k]), __fmul_rn(omt, q1[k]));
-}
-
 // Coordinate of point k of an edge from its endpoint coordinates (a1, a2),
 // under a discretisation rule (see csd_capi.h).
 __device__ __forceinline__ float edge_coord(float a1, float a2, int64_t np, int mode, int64_t k) {
@@ -86,35 +81,6 @@ __device__ __forceinline__ float edge_coord(float a1, float a2, int64_t np, int 
   return __fadd_rn(__fmul_rn(t, a2), __fmul_rn(__fsub_rn(1.0f, t), a1));
 }
 
-// Point k of an edge under a discretisation rule (see csd_capi.h).
-__device__ __forceinline__ void edge_point(const float* q1, const float* q2, int d, int64_t np, int mode, int64_t k,
-                                           float* out) {
-  if (mode == CSD_EDGE_L2_REF) {
-    float t = __double2float_rn(__ddiv_rn((double)k, (double)np));
-    lerp_point(q1, q2, d, t, out);
-  } else if (mode == CSD_EDGE_LINF) {
-    int64_t T = np - 1;
-    if (T == 0) {
-      for (int i = 0; i < d; ++i) out[i] = q1[i];
-    } else {
-      float t = __double2float_rn(__ddiv_rn((double)k, (double)T));
-      lerp_point(q1, q2, d, t, out);
-    }
-  } else {
-    if (k == 0) {
-      for (int i = 0; i < d; ++i) out[i] = q1[i];
-    } else if (k == 1) {
-      for (int i = 0; i < d; ++i) out[i] = q2[i];
-    } else {
-      float ts = __double2float_rn(__ddiv_rn(1.0, (double)(np - 1)));
-      lerp_point(q1, q2, d, __fmul_rn(ts, (float)(k - 1)), out);
-    }
-  }
-}
-
-// One warp per edge, edges taken from a work counter. Points are visited
-// coarse to fine: with G = ceil(n/32), the visit order is g, G+g, 2G+g, ...
-// for g = 0, 1, ..., so the first 32 visits sample the whole edge evenly.
 // Pair index e of the upper triangle (i < j, row-major) of n nodes -> (i, j):
 // e = i n - i (i + 1) / 2 + (j - i - 1). The double-precision estimate of i
 // is corrected with exact integer row starts.
@@ -129,6 +95,9 @@ static __device__ __forceinline__ void edge_pair(int64_t e, int64_t n, int64_t* 
   *j = e - row_start(r) + r + 1;
 }
 
+// One warp per edge, edges taken from a work counter. Points are visited
+// coarse to fine: with G = ceil(n/32), the visit order is g, G+g, 2G+g, ...
+// for g = 0, 1, ..., so the first 32 visits sample the whole edge evenly.
 // nodes > 0: the edges are every pair i < j of the `nodes` configurations in
 // `starts` (ends unused), in upper-triangle row-major order.
 template <int M>

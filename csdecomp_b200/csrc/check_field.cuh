@@ -24,8 +24,9 @@
 // Work here is per moving geometry, about one cell read each: 1.65 ms (10^6
 // uniform configurations 5.6 -> 1.1 ms, 40,009 edges 18.2 -> 2.9 ms). Still
 // bound by instruction issue and by the latency of dependent loads, not by
-// bandwidth. Cells of at most 2^18 per plant (4 MB): the radius plus half a
-// cell diagonal bounds a list, so finer cells list little less.
+// bandwidth. Cells of at most 2^18 per plant (4 MB, and as much for their
+// lists): the radius plus half a cell diagonal bounds a list, so finer cells
+// list little less.
 #pragma once
 #include <cuda_fp16.h>
 

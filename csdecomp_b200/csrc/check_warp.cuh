@@ -13,8 +13,8 @@ namespace csd {
 // the broad phase is on: a free configuration of the 7-DOF arm in 200
 // primitives costs 1.6 ns there against 9.5 ns with the link-sphere
 // broad phase. The other two are the pair sweep of check_core.cuh, for plants
-// with moving boxes, more than 1,024 statics or the broad phase switched off
-// (every pair tested): statics staged in shared memory, or read from global
+// with moving boxes, more than 1,024 statics, geometry that build_field leaves
+// out, or the broad phase switched off (every pair tested): statics staged in shared memory, or read from global
 // memory when they do not fit.
 enum : int { kModeGlobal = 0, kModeStaged = 1, kModeField = 2 };
 

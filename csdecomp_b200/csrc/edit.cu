@@ -8,7 +8,8 @@
 // Eigen loop that tests every candidate against all faces so far.
 //
 // Here the editing is two launches after one upload:
-//   1. edit_bisect_kernel   one warp per collision: projection onto its own
+//   1. edit_bisect_kernel   one warp per collision (or a few collisions, where
+//                            there are more than warps): projection onto its own
 //                            segment, every bisection step a fused FK +
 //                            collision check of the midpoint, distance to the
 //                            projection (the EI-ZO bisection body,
@@ -229,7 +230,7 @@ csd_status_t csd_edit_regions(csd_plant_t plant, const float* collisions, const 
   }
   const VoxArgs va = vox_args(vtab_dev);
 
-  // 1. bisection, one warp per collision
+  // 1. bisection
   const int K = (int)n, steps = (int)options->bisection_steps;
   s = with_mode(plant_mode(plant), [&](auto md) -> csd_status_t {
     constexpr int M = decltype(md)::value;

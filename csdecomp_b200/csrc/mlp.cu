@@ -6,8 +6,8 @@
 //   * mlp_forward_kernel: one CTA per 128 rows of one net; the three hidden
 //     layers are chained through shared memory (the epilogue of layer l
 //     writes relu(acc + b) as bf16 straight into the K-major operand tile of
-//     layer l + 1), weights stream in 64-wide K chunks through a double
-//     buffer, the accumulator (128 x 256 f32) lives in TMEM. The 256 -> 1
+//     layer l + 1), weights stream in 32-wide K chunks through four stages
+//     of asynchronous copies, the accumulator (128 x 256 f32) lives in TMEM. The 256 -> 1
 //     output is a dot product in the last epilogue.
 //   * gemm_kernel<NT>: grouped D = A * B^T (both K-major bf16 in global
 //     memory) for the backward pass, with epilogues that store f32, or apply

@@ -53,8 +53,8 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // coordinates (scaled by in_scale, zero padded to 16) or, for training, bf16
 // rows already padded (xb).
 struct FwdGroup {
-  const float* x;   // [rows][dim] f32, or null when xb is used
-  const bf16* xb;   // [rows][16] bf16
+  const float* x;   // [rows][dim] f32, read where xb is null (training groups: what xb was converted from)
+  const bf16* xb;   // [rows][16] bf16, or null
   int rows, dim, net;
   float* logits;    // [rows]
   // training outputs (optional): transposed bf16 copies, leading dimension ld_t

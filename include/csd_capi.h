@@ -279,7 +279,10 @@ csd_status_t csd_eizo(csd_plant_t plant, const float* line_start, const float* l
  * inflations, each with its own plant (one of `plants`, which must outlive the
  * batch), segment and domain, advance together through one persistent kernel
  * per stage, replayed as a CUDA graph. Each slot computes exactly what
- * csd_inflator_inflate computes for the same inputs. No voxels. */
+ * csd_inflator_inflate computes for the same inputs. No voxels. All plants of a
+ * batch are checked one way: through their grids (csd_plant_set_culling) when
+ * every one of them has one, by the pair sweep otherwise (about four times the
+ * time), so plants that need the sweep are better kept in a batch of their own. */
 typedef struct csd_batch_s* csd_batch_t;
 /* csd_mlp_t (the surrogate bank, functions csd_mlp_* below) is declared above csd_check_edges_ranked. */
 csd_status_t csd_batch_create(const csd_plant_t* plants, int32_t num_plants, int32_t max_slots,
@@ -466,8 +469,9 @@ csd_status_t csd_quotient_probe(const float* s, int64_t ns, const float* a, int6
 /* Broad phase of the collision checks (no counterpart in the reference, which
  * tests every pair): pairs apart by more than 1e-4 m are skipped, found through
  * a grid over the statics and capsules around the links or, for plants with
- * moving boxes, through bounding spheres of links and statics. Verdicts are
- * unchanged. On by default for plants with at most 32 moving links and 1024
+ * moving boxes (or extents of hundreds of metres, numbers that are not finite,
+ * a moving geometry that reaches most of many statics at once), through
+ * bounding spheres of links and statics. Verdicts are unchanged. On by default for plants with at most 32 moving links and 1024
  * static geometries; enable = 0 evaluates every pair (the full sweep that
  * csd_plant_flops counts). Takes effect for later calls and for batches
  * created afterwards. */
