@@ -312,7 +312,7 @@ def roofline_point_check(csd, scene, torch, dev, flush):
 # DRAM bytes per launch from ncu captures (profiles/): the full-sweep checker
 # launch (2^20 configurations) and the sampler's launches of one 256-slot step.
 CHECKER_TRAFFIC_BYTES = 29.5e6
-SAMPLER_TRAFFIC_BYTES_PER_STEP = 216.4e6   # 147 launches, 156.5 MB read + 60.0 MB written
+SAMPLER_TRAFFIC_BYTES_PER_STEP = 160.6e6   # 148 launches, 113.1 MB read + 47.5 MB written
 
 
 def check_workloads(csd, torch, dev, flush, cpu: bool):
@@ -584,8 +584,9 @@ def main():
                                           "launches of one timed step, one ncu capture "
                                           "(profiles/batch_sample_kernel_dram_traffic_one_step.md); step basis, "
                                           "as achieved",
-                        "kernel": "batch_sample_kernel (hit-and-run, G lanes per chain, faces staged in shared memory; "
-                                  "autotuned variant " + tuned_plain["sample_variant"] + "; regions beyond its "
+                        "kernel": "batch_sample_regs_kernel (hit-and-run, face pairs in registers: regions of more than 8 "
+                                  "dimensions and 65 to 1,024 pairs) and batch_sample_kernel (G lanes per chain, faces "
+                                  "staged in shared memory; autotuned variant " + tuned_plain["sample_variant"] + "; regions beyond its "
                                   "staging: " + tuned_plain["large_region_variant"] + ")",
                         "flop_per_unit": batched.SAMPLE_FLOP_RULE,
                         "flop_per_step": s_flop, "kernel_ms_per_step": s_ms,
