@@ -19,10 +19,12 @@ constexpr double kProbeGrowth = 1.2;     // a probe's radius over its capsule's,
 constexpr int kMaxProbes = 12;           // probes of one capsule
 constexpr size_t kFieldStaticShared = 2048;  // static shared memory of a checking kernel, at most (a plant, work items)
 // Largest coordinates (metres from the world's origin) of a grid's box and of a
-// static's extents: up to there the FP32 rounding of a probe's place in its cell
-// (4 ulp of 128 m on each axis) and of a distance to a static (2 ulp of 256 m)
-// stay below kFieldMargin together.
-constexpr double kFieldGridLimit = 64, kFieldStaticLimit = 256;
+// static's extents, and longest side of the box: up to there the FP32 rounding
+// of a cell's centre (1 ulp of 128 m on each axis), of a probe's place in its
+// cell (4 ulp of 64 m) and of a distance to a static (3 ulp of 128 m) stay below
+// kFieldMargin together. On a rail (no bound on the reach) the box ends kFieldRail
+// from the origin.
+constexpr double kFieldGridLimit = 128, kFieldGridSide = 128, kFieldRail = 64, kFieldStaticLimit = 256;
 
 struct FieldBuild {
   const float4* statics;  // WG poses
@@ -351,11 +353,12 @@ csd_status_t build_field(csd_plant_s* h, const std::vector<FkJoint>& fk, const s
       const double pad = max_r * (1 + 1e-6) + 1e-3;
       f.far_lo[k] = (float)(static_box[k] - pad);
       f.far_hi[k] = (float)(static_box[3 + k] + pad);
-      // (a prismatic joint's reach has no bound: its grid ends at the limit, and probes beyond test every static)
-      lo[k] = std::max((double)f.far_lo[k], reach_box[k] < -1e299 ? -kFieldGridLimit : reach_box[k]);
-      hi[k] = std::max(lo[k] + 1e-3,
-                       std::min((double)f.far_hi[k], reach_box[3 + k] > 1e299 ? kFieldGridLimit : reach_box[3 + k]));
-      if (lo[k] < -kFieldGridLimit || hi[k] > kFieldGridLimit) return CSD_OK;
+      const bool rail = reach_box[k] < -1e299;  // a prismatic joint: probes beyond the grid test every static
+      lo[k] = std::max((double)f.far_lo[k], rail ? -kFieldRail : reach_box[k]);
+      hi[k] = std::min((double)f.far_hi[k], rail ? kFieldRail : reach_box[3 + k]);
+      if (rail && hi[k] <= lo[k]) return CSD_OK;
+      hi[k] = std::max(lo[k] + 1e-3, hi[k]);
+      if (lo[k] < -kFieldGridLimit || hi[k] > kFieldGridLimit || hi[k] - lo[k] > kFieldGridSide) return CSD_OK;
       vol *= hi[k] - lo[k];
     }
     set_grid(std::max(std::cbrt(vol / kFieldCells), kFieldMinEdge));

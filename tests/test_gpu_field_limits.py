@@ -88,7 +88,7 @@ def test_verdicts_beside_a_ground_of_any_extent():
 
 
 @pytest.mark.parametrize("prismatic", [False, True])
-@pytest.mark.parametrize("base", [(40.0, 0, 0), (63.0, 1, 0), (70.0, 0, 0)])
+@pytest.mark.parametrize("base", [(40.0, 0, 0), (63.0, 1, 0), (70.0, 0, 0), (-90.0, 100.0, -60.0), (120.0, 0, 0), (127.5, 0, 0), (0, 200.0, 0)])
 def test_verdicts_far_from_the_origin(prismatic, base):
     statics = [(k, tuple(np.add(c, base)), *d) for k, c, *d in ORDINARY + [(S, (0.1, 0.15, 0.0), 0.05)]]
     plant = arm(statics, prismatic, base=base)
