@@ -18,7 +18,7 @@
 
 namespace csd {
 
-constexpr size_t kUniformStageBytes = 48 * 1024;
+constexpr size_t kUniformStageBytes = 48 * 1024 - 64;  // with the flag, what a block has without being asked for more
 // Floats of a row: coefficients, offsets, padded so that 8 consecutive rows fall on different banks.
 __host__ __device__ constexpr int uniform_stride(int nq) { return nq == 7 ? 36 : 4 * nq + 4; }
 // Coordinate pairs that the packed rows of a dimension hold.
@@ -169,17 +169,21 @@ __global__ void __launch_bounds__(256, NQ <= 4 ? 4 : 2)
   if (faces.thread(F)) return;  // chain_kernel's (uniform across the block)
   const float* Ap = A + (int64_t)f0 * dim;
   const float* bp = b + f0;
-  bool staged = (size_t)P * RS * sizeof(float) <= kUniformStageBytes;
+  const bool staged = (size_t)P * RS * sizeof(float) <= kUniformStageBytes;
+  // coefficients beyond kMaxCoeff: one division per face. (A flag in shared memory is known to be uniform; with the
+  // result of a block vote the compiler keeps the step loop ready for divergence, 4% of it.)
+  __shared__ int big;
+  if (threadIdx.x == 0) big = 0;
   if (staged) {
-    bool big = false;
+    __syncthreads();
     for (int i = threadIdx.x; i < 2 * P * MAXD; i += blockDim.x) {
       const int p = i / (2 * MAXD), k = (i >> 1) % MAXD, f = min(2 * p + (i & 1), F - 1);  // an odd count repeats its last face
       const float v = k < dim ? Ap[(int64_t)f * dim + k] : 0.f;
       sm[p * RS + 2 * k + (i & 1)] = v;
-      big = big || !(fabsf(v) <= kMaxCoeff);
+      if (!(fabsf(v) <= kMaxCoeff)) big = 1;
     }
     for (int i = threadIdx.x; i < 2 * P; i += blockDim.x) sm[(i >> 1) * RS + 2 * MAXD + (i & 1)] = bp[min(i, F - 1)];
-    staged = !__syncthreads_or(big);  // coefficients beyond kMaxCoeff: one division per face, from global memory
+    __syncthreads();
   }
   const int gl = threadIdx.x & (G - 1), ngroups = blockDim.x / G;
   const int npairs = (dim + 1) >> 1, JB = (npairs >> 1) + 1;
@@ -234,7 +238,7 @@ __global__ void __launch_bounds__(256, NQ <= 4 ? 4 : 2)
         s = f2_sub(*reinterpret_cast<const uint64_t*>(sm + p * RS + 2 * MAXD), ax);
       };
       float tmax = FLT_MAX, tmin = -FLT_MAX;
-      for (int pass = staged ? 0 : 1;; ++pass) {
+      for (int pass = staged && !big ? 0 : 1;; ++pass) {
         if (pass == 0) {
           ThetaBits tb = theta_bits_start();
           for (int p = gl; p < P; p += G) {
